@@ -62,18 +62,20 @@ __device__ __forceinline__ float kdiv(float a, float b, float y) {
 }
 
 // How the face-value and cell formulas divide.  xd: by an x/y spacing with
-// its power-of-two reciprocal r (or 0); zn/zs/zn2: by dzn(k), dzs(k),
-// dzn(k)+dzn(k+1).  DivIEEE divides as written; DivPlane (the tile engine)
-// holds the divisors and reciprocals of planes kc-1..kc+1 in registers and
-// uses kdiv, and with P2 (every x/y spacing a power of two) multiplies by r.
+// its table entry r; zn/zs/zn2: by dzn(k), dzs(k), dzn(k)+dzn(k+1).  DivIEEE
+// divides as written; DivPlane (the tile engine) holds the divisors and
+// reciprocals of planes kc-1..kc+1 in registers and uses kdiv.  Its x/y
+// quotients: kXPow2 multiplies by r (every x/y spacing a power of two), kXRecip
+// takes kdiv with r = RN(1/d) (the tables tile_tables makes), kXDiv is fdiv.
 // All forms give the IEEE quotient's bits.
+enum { kXDiv = 0, kXPow2 = 1, kXRecip = 2 };
 struct DivIEEE {
     __device__ __forceinline__ float xd(float a, float d, float r) const { return fdiv(a, d, r); }
     __device__ __forceinline__ float zn(const Geo &g, float a, int k) const { return a / g.dzn[k]; }
     __device__ __forceinline__ float zs(const Geo &g, float a, int k) const { return a / g.dzs[k]; }
     __device__ __forceinline__ float zn2(const Geo &g, float a, int k) const { return a / (g.dzn[k] + g.dzn[k + 1]); }
 };
-template <bool P2>
+template <int XD>
 struct DivPlane {
     float bn[3], yn[3], bs[3], ys[3], bn2[3], yn2[3];  // planes kc-1, kc, kc+1
     int kc;
@@ -89,7 +91,9 @@ struct DivPlane {
             yn2[d] = g.rdzn2[k];
         }
     }
-    __device__ __forceinline__ float xd(float a, float d, float r) const { return P2 ? a * r : fdiv(a, d, r); }
+    __device__ __forceinline__ float xd(float a, float d, float r) const {
+        return XD == kXPow2 ? a * r : (XD == kXRecip ? kdiv(a, d, r) : fdiv(a, d, r));
+    }
     __device__ __forceinline__ float zn(const Geo &, float a, int k) const {
         return kdiv(a, bn[k - kc + 1], yn[k - kc + 1]);
     }

@@ -191,12 +191,14 @@ struct les_ctx {
     bool uploaded = false;
     bool rhs_raw = false;  // interior of rhs holds values before the rhsav subtraction
     int red_gx = 0, red_gy = 0, red_nk = 0, red_kchunk = 0;
+    int nsm = 148;  // SMs of the context's device
     int last_n = 0;
     std::vector<float *> extra;      // scratch boxes of the per-routine entries
     const float *cn1_box = nullptr;  // caller's cn1 (per-routine press only)
     // temporal-blocked SOR (les_sor_tb.cuh)
     float *d_p2 = nullptr;           // second p buffer
     TbShape tb;  // SOR pass shape chosen by the autotuner (tb.T == 0: not yet)
+    bool xy_uni = false;   // every dx1 the same and every dy1 the same (build_tables)
     bool xy_pow2 = false;  // every x/y spacing divisor a power of two (build_tables)
     bool cn1_by_k = false;           // uniform dx, dy: cn1 from a per-k table
     bool p_ghosts_ok = false;        // p's ghosts hold what boundp1/boundp2 give
@@ -370,6 +372,9 @@ les_status build_tables(les_ctx *c, const les_host_fields *hf, bool require_infl
     for (int i = -1; i <= ip; ++i) c->xy_pow2 = c->xy_pow2 && h[t.rsx + i + 1] != 0.0f;
     for (int j = 0; j <= jp + 1; ++j) c->xy_pow2 = c->xy_pow2 && h[t.rdy1 + j] != 0.0f;
     for (int j = 0; j <= jp; ++j) c->xy_pow2 = c->xy_pow2 && h[t.rsy + j] != 0.0f;
+    c->xy_uni = true;
+    for (int i = 0; i <= ip + 1; ++i) c->xy_uni = c->xy_uni && dx1(i) == dx1(-1);
+    for (int j = 1; j <= jp + 1; ++j) c->xy_uni = c->xy_uni && dy1(j) == dy1(0);
     // grid-only denominator of rhsav and pav (press.f95:134, 192)
     i128 acc = 0;
     int bad = 0;
@@ -426,22 +431,46 @@ les_status enqueue_bondv1(les_ctx *c, int n, bool velnw) {
     return LES_OK;
 }
 
+// Planes per CTA of a momentum kernel whose grid holds `tiles` tiles of km
+// planes and `cap` CTAs at a time.  A CTA marches its planes one after the
+// other (3 to 6 us a plane), so a grid with few tiles is as slow as one
+// march; cutting the march fills the chip, at about three planes of set-up
+// per piece (two planes of face values, five of the band).  The cut with the
+// least waves x (planes + 3) is taken: one wave of 95 tiles becomes one of
+// 285 at 150 x 150 x 90 (k_mom1 563 -> 240 us, k_mom2 554 -> 207), 5 tiles
+// of 16 planes become 48 at 24 x 20 x 16 (70 -> 18 us each); at
+// 600 x 600 x 120 k_mom1 stays whole (5 x 123 plane steps against 10 x 63 or
+// 15 x 43) and k_mom2 takes 13 waves of 33 for 4 of 123 (1578 -> 1451 us).
+int mom_kchunk(int km, long long tiles, int cap) {
+    int best = km;
+    long long cost = -1;
+    for (int nz = 1; nz <= km; ++nz) {
+        const int kc = cdiv(km, nz);
+        const long long w = cdiv(tiles * cdiv(km, kc), cap) * (long long)(kc + 3);
+        if (cost < 0 || w < cost) cost = w, best = kc;
+    }
+    return best;
+}
+
 les_status enqueue_velfg_les(les_ctx *c, bool adam) {
     const Geo &g = c->geo;
-    const dim3 mg(cdiv(g.im, kMX), cdiv(g.jm, kMY));
+    const long long tiles = (long long)cdiv(g.im, kMX) * cdiv(g.jm, kMY);
+    const int kc1 = mom_kchunk(g.km, tiles, c->nsm * kMom1PerSM), kc2 = mom_kchunk(g.km, tiles, c->nsm * kMom2PerSM);
+    const dim3 mg(cdiv(g.im, kMX), cdiv(g.jm, kMY), cdiv(g.km, kc1));
+    const dim3 mg2(mg.x, mg.y, cdiv(g.km, kc2));
     const bool band = g.jm >= kBH;  // the staged band must not wrap onto itself
     const bool p2 = band && c->xy_pow2;
     if (p2)
-        LAUNCH_SMEM(c, (k_mom1<true, true>), mg, dim3(kMNT), mom_smem(false), g, c->F);
+        LAUNCH_SMEM(c, (k_mom1<true, true>), mg, dim3(kMNT), mom_smem(false), g, c->F, kc1, c->xy_uni);
     else if (band)
-        LAUNCH_SMEM(c, (k_mom1<true, false>), mg, dim3(kMNT), mom_smem(false), g, c->F);
+        LAUNCH_SMEM(c, (k_mom1<true, false>), mg, dim3(kMNT), mom_smem(false), g, c->F, kc1, c->xy_uni);
     else
-        LAUNCH_SMEM(c, (k_mom1<false, false>), mg, dim3(kMNT), mom_smem(false), g, c->F);
+        LAUNCH_SMEM(c, (k_mom1<false, false>), mg, dim3(kMNT), mom_smem(false), g, c->F, kc1, c->xy_uni);
     MARK(c, EV_VELFG);
     const long long nb = 2LL * (g.jm + 3) * (g.km + 2) + 2LL * g.im * (g.km + 2) + 2LL * g.im * (g.jm + 1);
     LAUNCH(c, k_boundsm, dim3(cdiv(nb, 256)), dim3(256), g, c->F.sm);
     const size_t sm2 = mom_smem(true);
-#define M2(A, B, P) LAUNCH_SMEM(c, (k_mom2<A, B, P>), mg, dim3(kMNT), sm2, g, c->F)
+#define M2(A, B, P) LAUNCH_SMEM(c, (k_mom2<A, B, P>), mg2, dim3(kMNT), sm2, g, c->F, kc2, c->xy_uni)
     if (adam) {
         if (p2)
             M2(true, true, true);
@@ -924,6 +953,12 @@ les_status les_ctx_create(const les_params *prm, les_ctx **out) {
     g.beta = prm->beta;
     g.omega = prm->omega;
     c->box_elems = (size_t)g.si * g.sj * g.sk;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        delete c;
+        return fail(LES_ERR_CUDA, "device attributes");
+    }
     auto cleanup = [&](les_status st) {
         const std::string msg = g_err;  // destroy resets the error string
         les_ctx_destroy(c);

@@ -21,6 +21,7 @@ namespace {  // kernels get internal linkage: each .cu has its own copy
 constexpr int kMX = 32, kMY = 8, kMNT = 352;
 constexpr int kMEX = kMX + 2, kMEY = kMY + 2, kMPOS = kMEX * kMEY;
 static_assert(kMNT % 32 == 0 && kMNT >= kMPOS && kMNT >= kMX * kMY, "one thread per ring position");
+constexpr int kMom1PerSM = 2, kMom2PerSM = 3;  // CTAs of k_mom1 / k_mom2 an SM holds (registers)
 enum { V_D1 = 0, V_C1 = 9, NV = 18 };
 
 // u, v, w staged in shared memory: a band of (32+4) x (8+4) columns/rows
@@ -46,15 +47,16 @@ struct UVWBand : DivIEEE {
     }
 };
 
-// The band for an interior tile: every position of the ring and its +-1
-// neighbours lies inside the band without moving by jm, and the plane slots
-// around the plane being filled (kc) are looked up once.
-template <bool P2>
-struct UVWBandFast : DivPlane<P2> {
+// The band read by position: row j - jb2 of the band is row j's real row
+// whether or not j lies in 1..jm, so a ring position and its +-1 neighbours
+// are read without moving by jm, and the plane slots around the plane being
+// filled (kc) are looked up once.
+template <int XD>
+struct UVWBandFast : DivPlane<XD> {
     const float *sl[4];  // slots of planes kc-1 .. kc+2
     int ib2, jb2;
     __device__ __forceinline__ UVWBandFast(const Geo &g, const float *base, int ib2_, int jb2_, int kc_)
-        : DivPlane<P2>(g, kc_), ib2(ib2_), jb2(jb2_) {
+        : DivPlane<XD>(g, kc_), ib2(ib2_), jb2(jb2_) {
         const int kc = kc_;
 #pragma unroll
         for (int d = 0; d < 4; ++d) sl[d] = base + ((kc + d) % kBS) * 3 * kBA;  // plane kc-1+d
@@ -262,15 +264,59 @@ __device__ __forceinline__ void vel2_pair_in(const Geo &g, const Q &q, int n, in
     }
 }
 
+// vel2_pair for a position of an edge tile of a grid whose x and y spacings
+// are uniform, from a band read by position: the values at (min(i, im), j),
+// kept where the array holds a computed value or a copy of one and 0
+// elsewhere.  For j = 0 and jm+1 the band's rows are those of the periodic
+// partner, whose spacings are the same, so the formula gives the copy's bits.
+// An edge tile so costs little more than an interior one; with the range
+// tests of vel2_pair and the moved rows of UVWBand a plane of it took twice an
+// interior tile's, 24% of the tiles at 300 x 300 and 46% at 150 x 150 (both
+// kernels together 447 -> 395 us at 150 x 150 x 90, 3464 -> 3202 us at
+// 600 x 600 x 120, the division by reciprocals of kXRecip included).
+// er: bit 0: 1 <= i <= im, 1: i == im+1, 2: 1 <= j <= jm, 3: j == 0, 4: j == jm+1.
+template <class Q>
+__device__ __forceinline__ void vel2_pair_edge(const Geo &g, const Q &q, int n, int i, int j, int k, int kr, int er,
+                                               float &d, float &c) {
+    const bool ii = er & 1, ie = er & 3, jj = er & 4, jp = er & 28;
+    vel2_pair_in(g, q, n, min(i, g.im), j, k, kr, d, c);
+    bool kd, kc;  // d, c kept
+    switch (n) {
+        case 1:
+        case 7: kd = kc = ie && jj; break;
+        case 2:
+            kc = ii && jp;
+            kd = kc || (ie && (er & 20));
+            break;
+        case 5:
+        case 8: kd = kc = ii && jp; break;
+        case 3:
+            kd = ie && jj;
+            kc = ii && jj;
+            break;
+        case 4:
+            kc = ie && jj;
+            kd = ie && (er & 12);
+            break;
+        case 6:
+            kc = ii && jj;
+            kd = ii && (er & 12);
+            break;
+        default: kd = kc = ii && jj; break;  // 9
+    }
+    d = kd ? d : 0.0f;
+    c = kc ? c : 0.0f;
+}
+
 // Shared-memory view: plane slots cur (k), nxt (k+1) and prv78 (diu7, diu8
 // of k-1), for the cell policies of les_step.cuh.
-template <bool P2>
-struct TileView : DivPlane<P2> {
+template <int XD>
+struct TileView : DivPlane<XD> {
     const float *cur, *nxt, *prv7, *prv8;
     int ib, jb, kc;  // i, j of ring position 0 and the current plane
     __device__ __forceinline__ TileView(const Geo &g, const float *cur_, const float *nxt_, const float *p7,
                                         const float *p8, int ib_, int jb_, int kc_)
-        : DivPlane<P2>(g, kc_), cur(cur_), nxt(nxt_), prv7(p7), prv8(p8), ib(ib_), jb(jb_), kc(kc_) {}
+        : DivPlane<XD>(g, kc_), cur(cur_), nxt(nxt_), prv7(p7), prv8(p8), ib(ib_), jb(jb_), kc(kc_) {}
     __device__ __forceinline__ int pos(int i, int j) const { return (j - jb) * kMEX + (i - ib); }
     __device__ __forceinline__ float dv(int n, int i, int j, int k) const {
         const int p = pos(i, j);
@@ -332,13 +378,18 @@ __device__ __forceinline__ void velfg_tile(const Geo &g, const TV &t, int i, int
 
 // Fill plane slot `dst` with the 18 values of plane k over the ring; copy
 // the diu7/diu8 the slot held (plane k-2) into prv7/prv8 first if asked.
-// INTERIOR: the whole ring lies in 1..im x 1..jm (see vel2_pair_in).
-template <bool DIU_ONLY, bool INTERIOR, class Q>
+// MODE: kTileIn, the whole ring lies in 1..im x 1..jm (vel2_pair_in);
+// kTileEdge, an edge tile of a uniform x/y grid (vel2_pair_edge); kTileAny.
+enum { kTileAny = 0, kTileIn = 1, kTileEdge = 2 };
+template <bool DIU_ONLY, int MODE, class Q>
 __device__ __forceinline__ void tile_plane(const Geo &g, const Q &q, float *dst, float *prv7, float *prv8, int ib,
                                            int jb, int k, bool save_prev) {
     const int kr = (k >= 1 && k <= g.km ? 1 : 0) | (k >= 1 && k <= g.km + 1 ? 2 : 0) | (k >= 1 && k <= g.km - 1 ? 4 : 0);
     for (int p = threadIdx.x; p < kMPOS; p += kMNT) {
         const int i = ib + p % kMEX, j = jb + p / kMEX;
+        const int er = MODE != kTileEdge ? 0
+                                         : (i >= 1 && i <= g.im ? 1 : 0) | (i == g.im + 1 ? 2 : 0) |
+                                               (j >= 1 && j <= g.jm ? 4 : 0) | (j == 0 ? 8 : 0) | (j == g.jm + 1 ? 16 : 0);
         if (save_prev) {
             prv7[p] = dst[(V_D1 + 6) * kMPOS + p];
             prv8[p] = dst[(V_D1 + 7) * kMPOS + p];
@@ -346,8 +397,10 @@ __device__ __forceinline__ void tile_plane(const Geo &g, const Q &q, float *dst,
 #pragma unroll
         for (int n = 1; n <= 9; ++n) {
             float d, c;
-            if (INTERIOR)
+            if (MODE == kTileIn)
                 vel2_pair_in(g, q, n, i, j, k, kr, d, c);
+            else if (MODE == kTileEdge)
+                vel2_pair_edge(g, q, n, i, j, k, kr, er, d, c);
             else
                 vel2_pair(g, q, n, i, j, k, d, c);
             dst[(V_D1 + n - 1) * kMPOS + p] = d;
@@ -440,18 +493,31 @@ __device__ __forceinline__ void visc_tile(const Geo &g, const TV &d, const ViscV
 // loaded there arrive while the plane's face values are being filled.
 // The x and y tables a tile reads (dx1, rdx1, rsx at i = ib-1 .. ib+kMEX,
 // dy1, rdy1, rsy at j = jb-1 .. jb+kMEY), copied into shared memory at the
-// start of an interior tile's march; the Geo the march hands on points its
-// x/y tables there (same values, read from shared instead of global memory).
+// start of the march; the Geo the march hands on points its x/y tables there
+// (same values, read from shared instead of global memory).  With kXRecip the
+// reciprocal tables are RN(1/d) of every divisor (0 outside kdiv's range),
+// for kdiv.  Indices outside the grid's tables (edge tiles, uniform spacings)
+// read the nearest entry.
 constexpr int kTabX = kMEX + 2, kTabY = kMEY + 2;
+template <int XD>
 __device__ __forceinline__ void tile_tables(const Geo &g0, Geo &g, float *tab, int ib, int jb) {
-    const float *srcx[3] = {g0.dx1, g0.rdx1, g0.rsx}, *srcy[3] = {g0.dy1, g0.rdy1, g0.rsy};
     for (int t = threadIdx.x; t < 3 * kTabX + 3 * kTabY; t += blockDim.x) {
-        if (t < 3 * kTabX)
-            tab[t] = srcx[t / kTabX][ib - 1 + t % kTabX];
+        const bool x = t < 3 * kTabX;
+        const int u = x ? t : t - 3 * kTabX, w = x ? u / kTabX : u / kTabY;
+        const float *d1 = x ? g0.dx1 : g0.dy1, *r1 = x ? g0.rdx1 : g0.rdy1, *rs = x ? g0.rsx : g0.rsy;
+        const int lo = x ? -1 : 0, hi = (x ? g0.im : g0.jm) + 1;
+        const int q0 = x ? ib - 1 + u % kTabX : jb - 1 + u % kTabY;
+        const int q = min(max(q0, lo), w == 2 ? hi - 1 : hi);
+        float v;
+        if (w == 0)
+            v = d1[q];
+        else if (XD != kXRecip)
+            v = (w == 1 ? r1 : rs)[q];
         else {
-            const int u = t - 3 * kTabX;
-            tab[t] = srcy[u / kTabY][jb - 1 + u % kTabY];
+            const float d = w == 1 ? d1[q] : d1[q] + d1[q + 1], m = fabsf(d);
+            v = (m >= 0x1p-30f && m <= 0x1p30f) ? 1.0f / d : 0.0f;
         }
+        tab[t] = v;
     }
     g = g0;
     g.dx1 = tab - (ib - 1);
@@ -462,8 +528,9 @@ __device__ __forceinline__ void tile_tables(const Geo &g0, Geo &g, float *tab, i
     g.rsy = tab + 3 * kTabX + 2 * kTabY - (jb - 1);
 }
 
-template <bool DIU_ONLY, bool BAND, bool INTERIOR, bool P2, class PreFn, class CellFn>
-__device__ __forceinline__ void mom_march(const Geo &g0, const Fields &F, PreFn pre, CellFn cell) {
+// XD: the tile's x/y quotients (kXDiv in kTileAny, whose Geo keeps the global tables).
+template <bool DIU_ONLY, bool BAND, int MODE, int XD, class PreFn, class CellFn>
+__device__ __forceinline__ void mom_march(const Geo &g0, const Fields &F, int kc, PreFn pre, CellFn cell) {
     extern __shared__ float sh[];
     __shared__ float tabs[3 * kTabX + 3 * kTabY];
     constexpr int NVU = DIU_ONLY ? 9 : NV;
@@ -473,25 +540,27 @@ __device__ __forceinline__ void mom_march(const Geo &g0, const Fields &F, PreFn 
     float *band = prv8 + kMPOS;
     const int i0 = 1 + blockIdx.x * kMX, j0 = 1 + blockIdx.y * kMY;
     const int ib = i0 - 1, jb = j0 - 1;
+    const int ks = 1 + blockIdx.z * kc, ke = min(g0.km, ks + kc - 1);  // this CTA's planes
     Geo gl;
-    if (BAND && INTERIOR)
-        tile_tables(g0, gl, tabs, ib, jb);  // read after the first barrier below
+    constexpr bool kTab = BAND && MODE != kTileAny;
+    if (kTab)
+        tile_tables<XD>(g0, gl, tabs, ib, jb);  // read after the first barrier below
     else
         gl = g0;
     const Geo &g = gl;
     const UVW qg{{}, F.u, F.v, F.w};
     const UVWBand qb{{}, band, i0 - 2, j0 - 2};
     auto fill = [&](float *dst, int k, bool save) {
-        if (BAND && INTERIOR)
-            tile_plane<DIU_ONLY, true>(g, UVWBandFast<P2>(g, band, i0 - 2, j0 - 2, k), dst, prv7, prv8, ib, jb, k, save);
+        if (kTab)
+            tile_plane<DIU_ONLY, MODE>(g, UVWBandFast<XD>(g, band, i0 - 2, j0 - 2, k), dst, prv7, prv8, ib, jb, k, save);
         else if (BAND)
-            tile_plane<DIU_ONLY, false>(g, qb, dst, prv7, prv8, ib, jb, k, save);
+            tile_plane<DIU_ONLY, kTileAny>(g, qb, dst, prv7, prv8, ib, jb, k, save);
         else
-            tile_plane<DIU_ONLY, false>(g, qg, dst, prv7, prv8, ib, jb, k, save);
+            tile_plane<DIU_ONLY, kTileAny>(g, qg, dst, prv7, prv8, ib, jb, k, save);
     };
     const BandCopies bc = BAND ? BandCopies(g, F, i0 - 2, j0 - 2) : BandCopies();
-    if (BAND) {  // planes -1..1 and 0..2 fill the first two face planes
-        for (int k = -1; k <= 2; ++k) bc.load(band, k);
+    if (BAND) {  // planes ks-2..ks and ks-1..ks+1 fill the first two face planes
+        for (int k = ks - 2; k <= ks + 1; ++k) bc.load(band, k);
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
@@ -510,7 +579,7 @@ __device__ __forceinline__ void mom_march(const Geo &g0, const Fields &F, PreFn 
             cp_async4(dst + p, F.sm + IX(g, ib + p % kMEX, jb + p / kMEX, kk));
     };
     // A and B of plane kk from its staged sm (les.f95:179-185 inner terms)
-    auto plane_ab = [&](const DivPlane<P2> &dv, int kk, bool with_b) {
+    auto plane_ab = [&](const DivPlane<XD> &dv, int kk, bool with_b) {
         const float *S = sm_slot(kk);
         float *A = vA + (kk & 1) * kMPOS, *B = vB + (kk & 1) * kMPOS;
         for (int p = threadIdx.x; p < kMPOS; p += kMNT) {
@@ -521,25 +590,26 @@ __device__ __forceinline__ void mom_march(const Geo &g0, const Fields &F, PreFn 
         }
     };
     if (DIU_ONLY) {
-        stage_sm(0);
-        stage_sm(1);
-        stage_sm(2);
+        stage_sm(ks - 1);
+        stage_sm(ks);
+        stage_sm(ks + 1);
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
-        const DivPlane<P2> d0(g, 0), d1(g, 1);
-        plane_ab(d0, 0, false);
-        plane_ab(d1, 1, true);
+        const DivPlane<XD> d0(g, ks - 1), d1(g, ks);
+        plane_ab(d0, ks - 1, false);
+        plane_ab(d1, ks, true);
         __syncthreads();
-        const float *A0 = vA, *A1 = vA + kMPOS;
+        const float *A0 = vA + ((ks - 1) & 1) * kMPOS, *A1 = vA + (ks & 1) * kMPOS;
+        float *XZ = vXZ + ((ks - 1) & 1) * kMPOS;
         for (int p = threadIdx.x; p < kMPOS; p += kMNT)
-            vXZ[p] = d0.zn2(g, g.dzn[1] * A0[p] + g.dzn[0] * A1[p], 0);
+            XZ[p] = d0.zn2(g, g.dzn[ks] * A0[p] + g.dzn[ks - 1] * A1[p], ks - 1);
     }
-    fill(s0, 0, false);
-    fill(s1, 1, false);
+    fill(slot((ks - 1) & 1), ks - 1, false);
+    fill(slot(ks & 1), ks, false);
     __syncthreads();
-    if (BAND) {  // plane 3 (needed at k = 1) takes the slot of plane -1, free after the fills
-        bc.load(band, 3);
+    if (BAND) {  // plane ks+2 (needed at k = ks) takes the slot of plane ks-2, free after the fills
+        bc.load(band, ks + 2);
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
@@ -547,18 +617,18 @@ __device__ __forceinline__ void mom_march(const Geo &g0, const Fields &F, PreFn 
     // In the march, plane k+3 goes into the slot of plane k-1, whose last
     // reader (the fill of plane k at step k-1) finished before the barrier
     // that ends step k-1.
-    for (int k = 1; k <= g.km; ++k) {
+    for (int k = ks; k <= ke; ++k) {
         pre(k);
         if (BAND) {  // plane k+3 streams in while plane k+1 is filled from k..k+2
-            if (k + 3 <= g.km + 2) bc.load(band, k + 3);
+            if (k + 3 <= ke + 2) bc.load(band, k + 3);
             cp_async_commit();
         }
         // slot (k+1)&1 holds plane k-1: keep its diu7/diu8, then plane k+1
         fill(slot((k + 1) & 1), k + 1, true);
-        if (DIU_ONLY && k + 2 <= g.km + 1) stage_sm(k + 2);  // waited for with the band copies
+        if (DIU_ONLY && k + 2 <= ke + 1) stage_sm(k + 2);  // waited for with the band copies
         if (DIU_ONLY) cp_async_commit();
         __syncthreads();
-        const TileView<P2> t(g, slot(k & 1), slot((k + 1) & 1), prv7, prv8, ib, jb, k);
+        const TileView<XD> t(g, slot(k & 1), slot((k + 1) & 1), prv7, prv8, ib, jb, k);
         ViscView vv{};
         if (DIU_ONLY) {
             // A, B of plane k+1; exz, eyz between k and k+1; exy, fxy of k
@@ -597,9 +667,10 @@ __device__ __forceinline__ bool tile_interior_b(const Geo &g) {
 }
 #define tile_interior(g) tile_interior_b<BAND>(g)
 
-// velFG + feedbf + sgs viscosity (les.f95:132-152) for a 32 x 8 tile, all k.
+// velFG + feedbf + sgs viscosity (les.f95:132-152) for a 32 x 8 tile, kc planes.
+// uni: every dx1 and every dy1 the same, so an edge tile takes kTileEdge.
 template <bool BAND, bool P2>
-__global__ void __launch_bounds__(kMNT) k_mom1(Geo g, Fields F) {
+__global__ void __launch_bounds__(kMNT) k_mom1(Geo g, Fields F, int kc, bool uni) {
     const int i = 1 + blockIdx.x * kMX + threadIdx.x % kMX, j = 1 + blockIdx.y * kMY + threadIdx.x / kMX;
     const bool mine = threadIdx.x < kMX * kMY && i <= g.im && j <= g.jm;
     // the cell's own inputs of plane k (feedbf.f95:38-66, velFG's h), loaded
@@ -619,7 +690,7 @@ __global__ void __launch_bounds__(kMNT) k_mom1(Geo g, Fields F) {
         cm0 = __ldg(&F.cmask[c]);
         dm0 = __ldg(&F.dmask[c]);
     };
-    auto cell = [&](const Geo &g, const TileView<P2> &t, int k, const ViscView &) {
+    auto cell = [&](const Geo &g, const auto &t, int k, const ViscView &) {
         if (!mine) return;
         const int c = IX(g, i, j, k);
         float fv, gv, hv = h0;
@@ -646,16 +717,18 @@ __global__ void __launch_bounds__(kMNT) k_mom1(Geo g, Fields F) {
         F.sm[c] = sgs_sm(g, t, i, j, k);
     };
     if (tile_interior(g))
-        mom_march<false, BAND, true, P2>(g, F, pre, cell);
+        mom_march<false, BAND, kTileIn, P2 ? kXPow2 : kXRecip>(g, F, kc, pre, cell);
+    else if (BAND && uni)
+        mom_march<false, BAND, kTileEdge, P2 ? kXPow2 : kXRecip>(g, F, kc, pre, cell);
     else
-        mom_march<false, BAND, false, P2>(g, F, pre, cell);
+        mom_march<false, BAND, kTileAny, kXDiv>(g, F, kc, pre, cell);
 }
 
-// les.f95:170-274 viscous terms (+ adam.f95:32-46) for a 32 x 8 tile, all k.
+// les.f95:170-274 viscous terms (+ adam.f95:32-46) for a 32 x 8 tile, kc planes.
 // Three CTAs per SM (at most 62 registers, no spills): 1.91 -> 1.72 ms at
 // 600 x 600 x 120 (k_mom1 at three was slower, 2.16 -> 2.25 ms).
 template <bool ADAM, bool BAND, bool P2>
-__global__ void __launch_bounds__(kMNT, 3) k_mom2(Geo g, Fields F) {
+__global__ void __launch_bounds__(kMNT, 3) k_mom2(Geo g, Fields F, int kc, bool uni) {
     const int i = 1 + blockIdx.x * kMX + threadIdx.x % kMX, j = 1 + blockIdx.y * kMY + threadIdx.x / kMX;
     const bool mine = threadIdx.x < kMX * kMY && i <= g.im && j <= g.jm;
     // the cell's f, g, h (and fold, gold, hold) of plane k, loaded ahead by
@@ -673,7 +746,7 @@ __global__ void __launch_bounds__(kMNT, 3) k_mom2(Geo g, Fields F) {
             ho0 = F.hold[c];
         }
     };
-    auto cell = [&](const Geo &g, const TileView<P2> &t, int k, const ViscView &vv) {
+    auto cell = [&](const Geo &g, const auto &t, int k, const ViscView &vv) {
         if (!mine) return;
         float vfu, vfv, vfw;
         visc_tile(g, t, vv, i, j, k, vfu, vfv, vfw);
@@ -693,9 +766,11 @@ __global__ void __launch_bounds__(kMNT, 3) k_mom2(Geo g, Fields F) {
         }
     };
     if (tile_interior(g))
-        mom_march<true, BAND, true, P2>(g, F, pre, cell);
+        mom_march<true, BAND, kTileIn, P2 ? kXPow2 : kXRecip>(g, F, kc, pre, cell);
+    else if (BAND && uni)
+        mom_march<true, BAND, kTileEdge, P2 ? kXPow2 : kXRecip>(g, F, kc, pre, cell);
     else
-        mom_march<true, BAND, false, P2>(g, F, pre, cell);
+        mom_march<true, BAND, kTileAny, kXDiv>(g, F, kc, pre, cell);
 }
 
 }  // namespace
