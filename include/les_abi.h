@@ -127,6 +127,9 @@ les_status les_step(les_ctx *ctx, int n0, int nsteps);
 /* Replace the external inflow profile wind_profile(1:jp,1:kp) (host array)
  * before the next step (run_LES_kernel's per-step wind_profile argument). */
 les_status les_set_wind_profile(les_ctx *ctx, const float *wind_profile);
+/* Waits for the context's work.  LES_ERR_TIMEOUT (here, in les_last_metrics,
+ * les_ctx_download and les_ensemble_sync): a bounded wait between the thread
+ * blocks of a step's SOR gave up; the state is not that step's. */
 les_status les_ctx_sync(les_ctx *ctx);
 les_status les_last_metrics(les_ctx *ctx, les_metrics *m);
 /* The WV_DEBUG sums (velnw.f95:61-68, feedbf.f95:30-36,68-83, the sum(x)
@@ -173,7 +176,8 @@ enum { LES_RED_CANONICAL = 0, LES_RED_F_RHSAV = 1, LES_RED_F_SOR = 2, LES_RED_F_
        LES_RED_FAITHFUL = 7 };
 les_status les_ctx_set_reduction_mode(les_ctx *ctx, int mode);
 /* SOR iterations one SOR kernel launch of the next step carries: 0.5 for a
- * colour sweep, 2 for a multi-iteration pass. */
+ * colour sweep, 1 to 3 for a pass; 1 also for grids whose whole SOR runs in
+ * one launch with p on the chip (the pass shapes below then stay 0). */
 float les_ctx_sor_iters_per_launch(les_ctx *ctx);
 /* Iterations per pass and tile rows the autotuner chose for the
  * multi-iteration SOR (0, 0 before the first step that uses it). */

@@ -17,7 +17,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "liblesb200.so"
 CHECKED = PKG / "liblesb200_checked.so"
-SOURCES = ["les_lib.cu", "les_setup.cu", "les_noalloc.cu", "les_netcdf.cu"]
+SOURCES = ["les_lib.cu", "les_sor_res.cu", "les_sor_res_m.cu", "les_sor_res_l.cu", "les_setup.cu", "les_noalloc.cu", "les_netcdf.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 NVCC_FLAGS = [

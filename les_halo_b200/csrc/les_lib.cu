@@ -25,6 +25,7 @@
 #include "les_sor_tb.cuh"
 #include "les_sor1.cuh"
 #include "les_sor1p.cuh"
+#include "les_sor_res.cuh"
 #include "les_stats.cuh"
 #include "les_refine.cuh"
 #include "les_spectral.cuh"
@@ -34,6 +35,8 @@
 #include "les_dd.cuh"
 
 using namespace les;
+
+const void *les_res_kernel(int seg);  // les_sor_res.cu
 
 namespace {
 
@@ -200,6 +203,16 @@ struct les_ctx {
     TbShape tb;  // SOR pass shape chosen by the autotuner (tb.T == 0: not yet)
     bool xy_uni = false;   // every dx1 the same and every dy1 the same (build_tables)
     bool xy_pow2 = false;  // every x/y spacing divisor a power of two (build_tables)
+    // chip-resident SOR (les_sor_res.cuh), set up before the first step that can use it
+    ResPlan res;
+    bool res_tried = false;
+    ulonglong2 *d_ll = nullptr;
+    float4 *d_rg = nullptr;
+    float *d_resid = nullptr;
+    FixPart *d_respart = nullptr;
+    unsigned *d_resctl = nullptr;
+    int *h_reserr = nullptr, *d_reserr = nullptr;  // host-mapped: a bounded wait of it gave up
+    bool cn_uni = false;             // cn2l = cn2s and cn3l = cn3s, one value each
     bool cn1_by_k = false;           // uniform dx, dy: cn1 from a per-k table
     bool p_ghosts_ok = false;        // p's ghosts hold what boundp1/boundp2 give
     bool force_exact_sor = false;    // testing: always the per-colour path
@@ -242,6 +255,9 @@ namespace {
 float *field_ptr(les_ctx *c, int f) { return c->d_fields + (size_t)f * c->box_elems; }
 les_status launch_sor_tb(les_ctx *c, const TbShape &sh, int niter, int mode, float pjuge, int itmax,
                          bool tuning = false, const SorBufs *bufs = nullptr);
+les_status launch_sor_res(les_ctx *c);
+constexpr int kResIters = 4096;  // iterations its residual record holds
+constexpr size_t kResStatic = 2048;  // its static shared memory, at most
 
 // The SOR of the next step runs one colour sweep at a time (press.f95's own
 // sequence with materialised ghosts) instead of the temporal-blocked passes:
@@ -252,6 +268,13 @@ les_status launch_sor_tb(les_ctx *c, const TbShape &sh, int niter, int mode, flo
 bool sor_per_colour(const les_ctx *c) {
     return c->force_exact_sor || ((c->prm.jp % 2) != 0 && c->prm.jp < tb_rh(1, 4)) || !c->p_ghosts_ok ||
            c->prm.kp >= kTbKMax || (c->red_mode & LES_RED_F_SOR);
+}
+
+// The SOR of the next step runs in one launch with p on the chip
+// (les_sor_res.cuh): wherever it fits and the passes would run, unless
+// LES_SOR_TILE asks for a pass shape.
+bool sor_resident(const les_ctx *c) {
+    return !sor_per_colour(c) && !c->dd && c->res.seg && c->cn1_by_k && c->cn_uni && c->prm.omega == 1.0f && c->prm.nmaxp >= 1 && c->prm.nmaxp <= kResIters;
 }
 
 void drop_step_graphs(les_ctx *c) {
@@ -338,6 +361,12 @@ les_status build_tables(les_ctx *c, const les_host_fields *hf, bool require_infl
         c->cn1_by_k = uni && hf->dxs && hf->dys && hf->dzs;
         for (int k = 1; k <= kp; ++k) h[t.cn1k + k] = 1.0f / (h[t.cnA] + h[t.cnB] + h[t.cnC + k - 1]);
     }
+    // the x and y Poisson coefficients the same for every column, l and s alike
+    c->cn_uni = hf->cn2l && hf->cn2s && hf->cn3l && hf->cn3s;
+    for (int i = 0; i < ip && c->cn_uni; ++i)
+        c->cn_uni = h[t.cn2l + i] == h[t.cn2l] && h[t.cn2s + i] == h[t.cn2l];
+    for (int j = 0; j < jp && c->cn_uni; ++j)
+        c->cn_uni = h[t.cn3l + j] == h[t.cn3l] && h[t.cn3s + j] == h[t.cn3l];
     c->kq = TbKCoef{};
     for (int k = 1; k <= kp && k < kTbKMax; ++k) {
         c->kq.c4l[k] = h[t.cn4l + k - 1];
@@ -539,6 +568,11 @@ les_status enqueue_press(les_ctx *c, bool exact) {
             else
                 LAUNCH(c, k_final_sor, dim3(1), dim3(1024), c->d_part, 2 * np, c->prm.pjuge, c->d_scal);
         }
+    } else if (sor_resident(c)) {
+        MARK(c, EV_SOR1_START);
+        les_status st = launch_sor_res(c);
+        if (st != LES_OK) return st;
+        MARK(c, EV_SOR1_END);
     } else {
         const int nmaxp = c->prm.nmaxp;
         for (int done = 0, pass = 0; done < nmaxp; ++pass) {
@@ -742,6 +776,135 @@ les_status set_tb_smem_attrs() {
 #undef S2A
     g_tb_dyn_max = lim;
     return LES_OK;
+}
+
+// Tiles and segments of the chip-resident SOR for an ip x jp x kp grid, or
+// seg = 0 when it does not fit nsm SMs of smem_max bytes.  The plan with the
+// least cost of a half-sweep is taken, in cycles: 15 + 2.25 SEG per warp (what
+// its instructions and shared-memory words take), at least 1500 when columns
+// are exchanged (the trip through L2), and 8 for each row and column of a tile's
+// edge.  Measured against every segment length: the plan taken is the fastest,
+// or within 2% of it, at 24 x 20 x 16 (16 planes: 114 us; 8: 135, 24: 130, 32:
+// 233), 61 x 47 x 35 (8: 159; 16: 178, 24: 206, 64: 300) and 150 x 150 x 90 (48:
+// 362; 24: 438, 32: 364, 64: 607).
+ResPlan res_plan(int ip, int jp, int kp, int nsm, size_t smem_max) {
+    ResPlan best;
+    double cost = 0.0;
+    for (int seg : {8, 16, 24, 32, 40, 48, 64}) {
+        const bool rg = seg > 48;
+        const int nseg = cdiv(kp, seg);
+        for (int ntj = 1; ntj <= nsm; ++ntj) {
+            const int tj = cdiv(jp, ntj);
+            if (cdiv(jp, tj) != ntj || (ntj > 1 && jp - (ntj - 1) * tj < 2)) continue;
+            for (int nti = 1; nti * ntj <= nsm; ++nti) {
+                const int ti = cdiv(ip, nti);
+                if (cdiv(ip, ti) != nti || (nti > 1 && ip - (nti - 1) * ti < 2)) continue;
+                ResPlan p;
+                const long long ncols = (long long)ti * tj;
+                if (ncols > 8192) continue;
+                p.rg = rg;
+                p.seg = seg, p.nseg = nseg, p.nti = nti, p.ntj = ntj, p.ti = ti, p.tj = tj;
+                p.warps = nseg * (cdiv((ncols + 1) / 2, 32) + cdiv(ncols / 2, 32));
+                if (p.warps < 2 || 32 * p.warps > res_threads(seg)) continue;
+                p.threads = 32 * p.warps;
+                p.pm = ((ti + 1) >> 1) + 1;
+                p.nc = p.pm * (tj + 2);
+                p.lch = (std::max(ti, tj) + 1) / 2;
+                p.smem = 4 * ((size_t)nseg * 2 * p.nc * (seg + 4) + (rg ? 0 : (size_t)p.threads * (seg + 4)) +
+                              3 * (size_t)nseg * seg + 2 * p.threads) +
+                         8 * (size_t)p.warps * kResList + 4 * 2 * (size_t)((ncols + 1) / 2 + 1);
+                if (p.smem > smem_max) continue;
+                p.ll_words = (size_t)p.ncta() * 4 * nseg * (seg / 4) * 2 * p.lch;
+                const double work = 200.0 + p.warps * (15.0 + (rg ? 2.4 : 2.25) * seg);
+                const double t = p.ncta() == 1 ? work : std::max(work, 1500.0) + 8.0 * (ti + tj);
+                if (!best.seg || t < cost) cost = t, best = p;
+            }
+        }
+    }
+    return best;
+}
+
+// Plan and buffers of the chip-resident SOR, once per context, before the
+// first step is captured.  A grid that does not fit keeps the passes.
+les_status res_setup(les_ctx *c) {
+    if (c->res_tried) return LES_OK;
+    c->res_tried = true;
+    int dev = 0, coop = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop || std::getenv("LES_SOR_TILE") || c->prm.nmaxp < 1 || c->prm.nmaxp > kResIters) return LES_OK;
+    int optin = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const ResPlan p = res_plan(c->prm.ip, c->prm.jp, c->prm.kp, c->nsm, (size_t)optin - kResStatic);
+    if (!p.seg) return LES_OK;
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, les_res_kernel(p.seg)));
+    if (p.smem + fa.sharedSizeBytes > (size_t)optin || p.threads > fa.maxThreadsPerBlock) return LES_OK;
+    CK(cudaFuncSetAttribute(les_res_kernel(p.seg), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            optin - (int)fa.sharedSizeBytes));
+    const int n = p.ncta();
+    if (cudaMalloc(&c->d_ll, 2 * p.ll_words * sizeof(ulonglong2)) != cudaSuccess ||
+        (p.rg && cudaMalloc(&c->d_rg, p.rg_words() * sizeof(float4)) != cudaSuccess) ||
+        cudaMalloc(&c->d_resid, sizeof(float) * (size_t)n * c->prm.nmaxp) != cudaSuccess ||
+        cudaMalloc(&c->d_respart, 2 * sizeof(FixPart) * (size_t)n) != cudaSuccess ||
+        cudaMalloc(&c->d_resctl, 3 * sizeof(unsigned)) != cudaSuccess ||
+        cudaHostAlloc(&c->h_reserr, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(LES_ERR_NOMEM, "buffers of the resident SOR");
+    }
+    *c->h_reserr = 0;
+    CK(cudaHostGetDevicePointer(&c->d_reserr, c->h_reserr, 0));
+    CK(cudaMemsetAsync(c->d_ll, 0, 2 * p.ll_words * sizeof(ulonglong2), c->stream));
+    CK(cudaMemsetAsync(c->d_resctl, 0, 3 * sizeof(unsigned), c->stream));
+    c->res = p;
+    return LES_OK;
+}
+
+les_status launch_sor_res(les_ctx *c) {
+    const ResPlan &p = c->res;
+    ResArgs a{};
+    a.p = c->F.p;
+    a.rhs = c->F.rhs;
+    a.ll = c->d_ll;
+    a.rg = c->d_rg;
+    a.resid = c->d_resid;
+    a.part = c->d_respart;
+    a.ctl = c->d_resctl;
+    a.err = c->d_reserr;
+    a.sc = c->d_scal;
+    a.c2 = c->h_tables[c->tl.cn2l];
+    a.c3 = c->h_tables[c->tl.cn3l];
+    a.itmax = c->prm.nmaxp;
+    a.exact0 = c->sor_fp32_test && c->prm.pjuge < 0x1p40f ? 0 : 1;
+    a.pjuge = c->prm.pjuge;
+    a.nti = p.nti, a.ntj = p.ntj, a.ti = p.ti, a.tj = p.tj, a.nseg = p.nseg;
+    a.pm = p.pm, a.nc = p.nc, a.lch = p.lch, a.warps = p.warps;
+    a.ll_slot = (int)p.ll_words;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.gridDim = dim3(p.ncta());
+    cfg.blockDim = dim3(p.threads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = c->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = p.ncta() > 1 ? 1 : 0;  // one CTA waits for nobody
+    void *args[] = {&c->geo, &a, &c->kq};
+    CK(cudaLaunchKernelExC(&cfg, les_res_kernel(p.seg), args));
+    ++c->launches;
+    return LES_OK;
+}
+
+// After a synchronisation: whether a bounded wait of the resident SOR gave
+// up in a step since the last call (p and what follows from it are then
+// not the step's).
+les_status res_check(les_ctx *c) {
+    if (!c->h_reserr || !*(volatile int *)c->h_reserr) return LES_OK;
+    *c->h_reserr = 0;
+    CK(cudaMemsetAsync(c->d_resctl, 0, 2 * sizeof(unsigned), c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return fail(LES_ERR_TIMEOUT, "SOR: a CTA waited for a neighbour's columns too long; the step is void");
 }
 
 // Process-wide cache of autotuned SOR pass shapes: (ip, jp, kp, SMs) -> shape.
@@ -1067,6 +1230,12 @@ les_status les_ctx_destroy(les_ctx *c) {
     cudaFree(c->d_part);
     cudaFree(c->d_stage);
     cudaFree(c->d_p2);
+    cudaFree(c->d_ll);
+    cudaFree(c->d_rg);
+    cudaFree(c->d_resid);
+    cudaFree(c->d_respart);
+    cudaFree(c->d_resctl);
+    if (c->h_reserr) cudaFreeHost(c->h_reserr);
     cudaFree(c->d_ave);
     cudaFree(c->d_p64);
     cudaFree(c->d_r32);
@@ -1233,6 +1402,7 @@ les_status les_ctx_download(les_ctx *c, les_host_fields *hf) {
         if ((s = download_field(c, f, dst[f])) != LES_OK) return s;
         CK(cudaStreamSynchronize(c->stream));
     }
+    if ((s = res_check(c)) != LES_OK) return s;
     if (hf->delx1) {
         for (int k = 1; k <= c->prm.kp; ++k) {
             const float *h = c->h_tables.data();
@@ -1303,6 +1473,7 @@ les_status les_ctx_sor_rows(les_ctx *c, int *rows) {
 float les_ctx_sor_iters_per_launch(les_ctx *c) {
     if (!c) return 0.0f;
     const bool exact = sor_per_colour(c);
+    if (!exact && sor_resident(c)) return 1.0f;
     return exact ? 0.5f : (float)(c->tb.T ? c->tb.T : 2);
 }
 
@@ -1370,7 +1541,13 @@ les_status les_step(les_ctx *c, int n0, int nsteps) {
         const int n = n0 + s;
         const bool exact = sor_per_colour(c);
         const int gi = ((n == 1 && c->prm.ical == 0) ? 1 : 0) + (exact ? 2 : 0);
-        if ((!exact || c->ref_outer > 0) && c->tb.T == 0) {  // the refined press uses the passes too
+        if (!exact && !c->res_tried) {
+            LES_RANGE("sor_autotune");
+            les_status st = res_setup(c);
+            if (st != LES_OK) return st;
+        }
+        // (the refined press uses the passes too)
+        if (((!exact && !sor_resident(c)) || c->ref_outer > 0) && c->tb.T == 0) {
             LES_RANGE("sor_autotune");
             les_status st = autotune_sor(c);
             if (st != LES_OK) return st;
@@ -1477,7 +1654,8 @@ les_status les_ctx_sync(les_ctx *c) {
     LES_RANGE("les_ctx_sync");
     if (!c) return fail(LES_ERR_BAD_ARG, "NULL ctx");
     CK(cudaStreamSynchronize(c->stream));
-    return ok();
+    les_status rs = res_check(c);
+    return rs == LES_OK ? ok() : rs;
 }
 
 les_status les_last_metrics(les_ctx *c, les_metrics *m) {
@@ -1486,6 +1664,7 @@ les_status les_last_metrics(les_ctx *c, les_metrics *m) {
     Scal s;
     CK(cudaMemcpyAsync(&s, c->d_scal, sizeof s, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (const les_status rs = res_check(c); rs != LES_OK) return rs;
     m->n = s.n;
     m->sor_iters = s.sor_iters;
     m->sor = s.sor;
