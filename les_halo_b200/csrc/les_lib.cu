@@ -211,7 +211,7 @@ struct les_ctx {
     float *d_resid = nullptr;
     FixPart *d_respart = nullptr;
     unsigned *d_resctl = nullptr;
-    int *h_reserr = nullptr, *d_reserr = nullptr;  // host-mapped: a bounded wait of it gave up
+    int *h_reserr = nullptr, *d_reserr = nullptr;  // host-mapped (res_err_take): a bounded wait of it gave up
     bool cn_uni = false;             // cn2l = cn2s and cn3l = cn3s, one value each
     bool cn1_by_k = false;           // uniform dx, dy: cn1 from a per-k table
     bool p_ghosts_ok = false;        // p's ghosts hold what boundp1/boundp2 give
@@ -824,6 +824,44 @@ ResPlan res_plan(int ip, int jp, int kp, int nsm, size_t smem_max) {
     return best;
 }
 
+// Host-mapped error words of the chip-resident SOR, one per context, from one
+// page-locked block per process (locking a page costs about a millisecond).
+// A process with more contexts alive than the block has words locks a page for
+// each of the others.
+constexpr int kResErrs = 1024;
+int *g_reserr = nullptr;
+unsigned char g_reserr_used[kResErrs] = {};
+std::mutex g_reserr_mu;
+bool res_err_take(les_ctx *c) {
+    {
+        std::lock_guard<std::mutex> lk(g_reserr_mu);
+        if (!g_reserr && cudaHostAlloc(&g_reserr, sizeof(int) * kResErrs,
+                                       cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            g_reserr = nullptr;
+            return false;
+        }
+        for (int q = 0; q < kResErrs && !c->h_reserr; ++q)
+            if (!g_reserr_used[q]) g_reserr_used[q] = 1, c->h_reserr = g_reserr + q;
+    }
+    if (!c->h_reserr && cudaHostAlloc(&c->h_reserr, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_reserr = nullptr;
+        return false;
+    }
+    *c->h_reserr = 0;
+    return cudaHostGetDevicePointer(&c->d_reserr, c->h_reserr, 0) == cudaSuccess;
+}
+void res_err_give(les_ctx *c) {
+    if (!c->h_reserr) return;
+    std::lock_guard<std::mutex> lk(g_reserr_mu);
+    if (c->h_reserr >= g_reserr && c->h_reserr < g_reserr + kResErrs)
+        g_reserr_used[c->h_reserr - g_reserr] = 0;
+    else
+        cudaFreeHost(c->h_reserr);
+    c->h_reserr = nullptr;
+}
+
 // Plan and buffers of the chip-resident SOR, once per context, before the
 // first step is captured.  A grid that does not fit keeps the passes.
 les_status res_setup(les_ctx *c) {
@@ -842,19 +880,24 @@ les_status res_setup(les_ctx *c) {
     if (p.smem + fa.sharedSizeBytes > (size_t)optin || p.threads > fa.maxThreadsPerBlock) return LES_OK;
     CK(cudaFuncSetAttribute(les_res_kernel(p.seg), cudaFuncAttributeMaxDynamicSharedMemorySize,
                             optin - (int)fa.sharedSizeBytes));
+    // one allocation (a new domain's first step pays for it): exchange words,
+    // rhs scratch, partial sums, residuals, control words
     const int n = p.ncta();
-    if (cudaMalloc(&c->d_ll, 2 * p.ll_words * sizeof(ulonglong2)) != cudaSuccess ||
-        (p.rg && cudaMalloc(&c->d_rg, p.rg_words() * sizeof(float4)) != cudaSuccess) ||
-        cudaMalloc(&c->d_resid, sizeof(float) * (size_t)n * c->prm.nmaxp) != cudaSuccess ||
-        cudaMalloc(&c->d_respart, 2 * sizeof(FixPart) * (size_t)n) != cudaSuccess ||
-        cudaMalloc(&c->d_resctl, 3 * sizeof(unsigned)) != cudaSuccess ||
-        cudaHostAlloc(&c->h_reserr, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+    const size_t ll = 2 * p.ll_words * sizeof(ulonglong2), rg = p.rg_words() * sizeof(float4),
+                 part = 2 * sizeof(FixPart) * (size_t)n, resid = sizeof(float) * (size_t)n * c->prm.nmaxp;
+    const size_t residp = (resid + 15) / 16 * 16;
+    char *base = nullptr;
+    if (cudaMalloc(&base, ll + rg + part + residp + 3 * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         return fail(LES_ERR_NOMEM, "buffers of the resident SOR");
     }
-    *c->h_reserr = 0;
-    CK(cudaHostGetDevicePointer(&c->d_reserr, c->h_reserr, 0));
-    CK(cudaMemsetAsync(c->d_ll, 0, 2 * p.ll_words * sizeof(ulonglong2), c->stream));
+    c->d_ll = reinterpret_cast<ulonglong2 *>(base);
+    c->d_rg = reinterpret_cast<float4 *>(base + ll);
+    c->d_respart = reinterpret_cast<FixPart *>(base + ll + rg);
+    c->d_resid = reinterpret_cast<float *>(base + ll + rg + part);
+    c->d_resctl = reinterpret_cast<unsigned *>(base + ll + rg + part + residp);
+    if (!res_err_take(c)) return fail(LES_ERR_NOMEM, "mapped word of the resident SOR");
+    CK(cudaMemsetAsync(c->d_ll, 0, ll, c->stream));
     CK(cudaMemsetAsync(c->d_resctl, 0, 3 * sizeof(unsigned), c->stream));
     c->res = p;
     return LES_OK;
@@ -1230,12 +1273,8 @@ les_status les_ctx_destroy(les_ctx *c) {
     cudaFree(c->d_part);
     cudaFree(c->d_stage);
     cudaFree(c->d_p2);
-    cudaFree(c->d_ll);
-    cudaFree(c->d_rg);
-    cudaFree(c->d_resid);
-    cudaFree(c->d_respart);
-    cudaFree(c->d_resctl);
-    if (c->h_reserr) cudaFreeHost(c->h_reserr);
+    cudaFree(c->d_ll);  // and d_rg, d_respart, d_resid, d_resctl
+    res_err_give(c);
     cudaFree(c->d_ave);
     cudaFree(c->d_p64);
     cudaFree(c->d_r32);
