@@ -25,10 +25,11 @@
 //     warps work meanwhile.  Two slots per word suffice: a CTA sends
 //     half-sweep s+2 only after it has received s+1 from the same neighbour
 //     column, which that column sent after it had read s.
-// What bounds it: at 150 x 150 x 90 a half-sweep takes 7.1 thousand cycles, of
-// which the edge warps' chain is all: 3.4 waiting for the neighbours' words (two
-// trips through L2), 2.5 of updates, 0.8 of sends; the other warps' updates, 3.1
-// (shared memory: 27 wavefronts per four updates of a warp), run beside it.
+// What bounds it: at 150 x 150 x 90 a half-sweep takes 7.1 thousand cycles, most
+// of it the edge warps' chain.  Clocked when a word was still polled before the
+// others were read (7.5 in all): 3.4 until the neighbours' words are there, 2.5
+// of updates, 0.8 of sends; the other warps' updates, 3.1 (shared memory: 27
+// wavefronts per four updates of a warp), run beside it.
 // With one CTA (24 x 20 x 16) nothing is exchanged and a half-sweep takes 2.2.
 // Measured, the SOR of a step (50 iterations), passes -> here: 24 x 20 x 16
 // 585 -> 117 us, 61 x 47 x 35 607 -> 162, 150 x 150 x 90 1226 -> 364,
