@@ -208,7 +208,7 @@ struct les_ctx {
     bool res_tried = false;
     ulonglong2 *d_ll = nullptr;
     float4 *d_rg = nullptr;
-    float *d_resid = nullptr;
+    u64 *d_resid = nullptr;
     FixPart *d_respart = nullptr;
     unsigned *d_resctl = nullptr;
     int *h_reserr = nullptr, *d_reserr = nullptr;  // host-mapped (res_err_take): a bounded wait of it gave up
@@ -796,7 +796,7 @@ ResPlan res_plan(int ip, int jp, int kp, int nsm, size_t smem_max) {
         for (int ntj = 1; ntj <= nsm; ++ntj) {
             const int tj = cdiv(jp, ntj);
             if (cdiv(jp, tj) != ntj || (ntj > 1 && jp - (ntj - 1) * tj < 2)) continue;
-            for (int nti = 1; nti * ntj <= nsm; ++nti) {
+            for (int nti = 1; nti * ntj <= std::min(nsm, kResCtas); ++nti) {
                 const int ti = cdiv(ip, nti);
                 if (cdiv(ip, ti) != nti || (nti > 1 && ip - (nti - 1) * ti < 2)) continue;
                 ResPlan p;
@@ -884,7 +884,7 @@ les_status res_setup(les_ctx *c) {
     // rhs scratch, partial sums, residuals, control words
     const int n = p.ncta();
     const size_t ll = 2 * p.ll_words * sizeof(ulonglong2), rg = p.rg_words() * sizeof(float4),
-                 part = 2 * sizeof(FixPart) * (size_t)n, resid = sizeof(float) * (size_t)n * c->prm.nmaxp;
+                 part = 2 * sizeof(FixPart) * (size_t)n, resid = sizeof(u64) * (size_t)((n + 1) & ~1) * c->prm.nmaxp;
     const size_t residp = (resid + 15) / 16 * 16;
     char *base = nullptr;
     if (cudaMalloc(&base, ll + rg + part + residp + 3 * sizeof(unsigned)) != cudaSuccess) {
@@ -894,10 +894,11 @@ les_status res_setup(les_ctx *c) {
     c->d_ll = reinterpret_cast<ulonglong2 *>(base);
     c->d_rg = reinterpret_cast<float4 *>(base + ll);
     c->d_respart = reinterpret_cast<FixPart *>(base + ll + rg);
-    c->d_resid = reinterpret_cast<float *>(base + ll + rg + part);
+    c->d_resid = reinterpret_cast<u64 *>(base + ll + rg + part);
     c->d_resctl = reinterpret_cast<unsigned *>(base + ll + rg + part + residp);
     if (!res_err_take(c)) return fail(LES_ERR_NOMEM, "mapped word of the resident SOR");
     CK(cudaMemsetAsync(c->d_ll, 0, ll, c->stream));
+    CK(cudaMemsetAsync(c->d_resid, 0, resid, c->stream));
     CK(cudaMemsetAsync(c->d_resctl, 0, 3 * sizeof(unsigned), c->stream));
     c->res = p;
     return LES_OK;
@@ -923,6 +924,7 @@ les_status launch_sor_res(les_ctx *c) {
     a.nti = p.nti, a.ntj = p.ntj, a.ti = p.ti, a.tj = p.tj, a.nseg = p.nseg;
     a.pm = p.pm, a.nc = p.nc, a.lch = p.lch, a.warps = p.warps;
     a.ll_slot = (int)p.ll_words;
+    a.rstride = (p.ncta() + 1) & ~1;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;

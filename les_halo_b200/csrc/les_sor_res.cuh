@@ -32,8 +32,8 @@
 // wavefronts per four updates of a warp), run beside it.
 // With one CTA (24 x 20 x 16) nothing is exchanged and a half-sweep takes 2.2.
 // Measured, the SOR of a step (50 iterations), passes -> here: 24 x 20 x 16
-// 585 -> 117 us, 61 x 47 x 35 607 -> 162, 150 x 150 x 90 1226 -> 364,
-// 257 x 203 x 61 1618 -> 690.  Packed two-wide FP32 instructions (18% fewer
+// 585 -> 119 us, 61 x 47 x 35 607 -> 162, 150 x 150 x 90 1226 -> 377,
+// 257 x 203 x 61 1618 -> 711.  Packed two-wide FP32 instructions (18% fewer
 // instructions) gave nothing, and need a -0 the assembler cannot see: it
 // contracts a packed multiply and add whatever --fmad says.
 //
@@ -44,13 +44,22 @@
 // half-sweep before they are read, which is the value press.f95 reads.
 //
 // Stop test: every iteration but the last sums reltmp^2 of one cell in four in
-// FP32 (no term is negative, so that is a lower bound of the whole sum) and is
-// checked at the end against the bound of tb_finish_fast (here at most SEG + 32
-// + 5 + 5 + 5 adds from a term to the root).  If some iteration's bound does
-// not rule the stop out, the loop runs again from the input p, which is
-// unchanged in memory until the loop ends, and from that iteration on sums
-// exactly (les_fix.h) and decides before it goes on.  Iteration counts, the
-// residual and p are those of exact sums throughout.
+// FP32 (no term is negative, so that is a lower bound of the whole sum), checked
+// against the bound of tb_finish_fast (here at most SEG + 32 + 5 + 5 + 5 adds
+// from a term to the root).  The CTAs exchange the bounds as words {value, tag}
+// and look at them while the loop runs, two iterations late, so that nobody waits;
+// after the first four iterations one word carries the least bound of four.
+// Where a look does not rule the stop out, all CTAs leave the attempt together
+// and the loop runs again from the input p, which is unchanged in memory until
+// it ends; from that batch on it sums exactly (les_fix.h) and decides before it
+// goes on.  A step that stops after m iterations so costs 2m + 3 to 2m + 8 of them
+// instead of the cap's (SOR of a step that stops after 10 of 50, looks at the end
+// -> while it runs; the passes: 24 x 20 x 16 167 -> 79 us; 220, 61 x 47 x 35
+// 235 -> 118; 235, 150 x 150 x 90 529 -> 271; 352, 257 x 203 x 61 927 -> 380; 440;
+// after 10 of 1000 at 150 x 150 x 90 6132 -> 272; 1428).  The looks cost 0 to 4.5%
+// of an SOR that runs to its cap (61 x 47 x 35 161 -> 162 us, 150 x 150 x 90
+// 363 -> 377, 257 x 203 x 61 681 -> 711) and nothing where no stop is asked for.
+// Iteration counts, the residual and p are those of exact sums throughout.
 //
 // Every wait is bounded: past kResPolls polls a thread gives up, the CTA
 // returns without writing p, and the context reports LES_ERR_TIMEOUT.
@@ -65,6 +74,13 @@ typedef unsigned long long u64;
 #define LES_INLINE __attribute__((always_inline))
 constexpr int kResPolls = 1 << 20;   // about a second
 constexpr int kResList = 64;         // halo columns of one warp (at most two per column)
+constexpr int kResCtas = 160;        // CTAs of a launch, at most
+// Batches of iterations whose FP32 bounds travel as one word: the first four
+// iterations one by one, then four each.
+constexpr int kResBatch = 4;
+__device__ __forceinline__ bool batch_ends(int l) { return l < kResBatch || l % kResBatch == kResBatch - 1; }
+__device__ __forceinline__ int batch_of(int l) { return l < kResBatch ? l : kResBatch - 1 + l / kResBatch; }
+__device__ __forceinline__ int batch_first(int l) { return l < kResBatch ? l : l / kResBatch * kResBatch; }
 
 struct ResPlan {
     int seg = 0, nseg = 0;           // planes per thread (0: no plan), segments per column
@@ -83,7 +99,7 @@ struct ResArgs {
     const float *rhs;
     ulonglong2 *ll;      // exchange words, two slots
     float4 *rg;          // rhs [CTA][parity, group][thread] (RG)
-    float *resid;        // FP32 residuals [iteration][CTA]
+    u64 *resid;          // FP32 bounds [batch of iterations][CTA], words {value, tag}
     FixPart *part;       // exact partial sums, two sets of one per CTA
     unsigned *ctl;       // [0] barrier arrivals, [1] barrier generation, [2] next tag
     int *err;            // host-mapped: a wait gave up
@@ -93,6 +109,7 @@ struct ResArgs {
     float pjuge;
     int nti, ntj, ti, tj, nseg, pm, nc, lch, warps;
     int ll_slot;         // words of one slot
+    int rstride;         // words of one batch in resid (even)
 };
 
 __device__ __forceinline__ void ll_store(ulonglong2 *dst, float v0, float v1, unsigned tag) {
@@ -106,6 +123,23 @@ __device__ __forceinline__ ulonglong2 ll_load(const ulonglong2 *src) {
     asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(src) : "memory");
     return v;
 }
+
+// A word {value, tag}: its tag says whose value it is.
+__device__ __forceinline__ void word_store(u64 *dst, float v, unsigned tag) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(dst), "l"((u64)tag << 32 | __float_as_uint(v)) : "memory");
+}
+__device__ __forceinline__ u64 word_load(const u64 *src) {
+    u64 w;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(w) : "l"(src) : "memory");
+    return w;
+}
+
+// Two words into shared memory, from L2, without waiting.
+__device__ __forceinline__ void word_fetch2(u64 *dst, const u64 *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void word_fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // All CTAs of the launch; true (in every thread) when the wait gave up.
 __device__ __forceinline__ bool res_grid_barrier(const ResArgs &a, int ncta, int *s_abort) {
@@ -143,7 +177,9 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
     k_sor_res(Geo g, ResArgs a, const __grid_constant__ TbKCoef kq) {
     constexpr int H = SEG / 2, NG = SEG / 8, NE = SEG / 4, CS = SEG + 4;
     extern __shared__ float4 rsm4[];
-    __shared__ int s_abort, s_cnt[4], s_stop;
+    __shared__ int s_abort, s_cnt[4], s_stop, s_look[2];
+    __shared__ float s_min;
+    __shared__ __align__(16) u64 s_words[kResCtas];
     Scal *const sc = a.sc;
     const int im = g.im, jm = g.jm, km = g.km, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int ncta = a.nti * a.ntj, cta = blockIdx.x, tx = cta % a.nti, ty = cta / a.nti;
@@ -175,7 +211,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
         if (side == 2) return y == 0 && !jself;
         return y == ny - 1 && !jself;
     };
-    if (tid == 0) s_abort = 0;
+    if (tid == 0) s_abort = 0, s_look[0] = s_look[1] = -1;
     // coefficient tables and zeroed columns (padded planes stay 0)
     for (int t = tid; t < a.nseg * 6 * H; t += blockDim.x) {
         const int q = t / (3 * H) % 2, w = t / H % 3, k = 1 + t / (6 * H) * SEG + 2 * (t % H) + q;
@@ -280,6 +316,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
     const unsigned tag0 = a.ctl[2];  // moved on after the last barrier of the launch
     unsigned tag = tag0;
     int exact_from = a.exact0 ? 0 : a.itmax - 1;
+    const bool stops = a.pjuge > 0.0f;  // (a sum of squares is not below 0)
     float P[2][H];  // the column's planes of each parity
 
     for (int attempt = 0;; ++attempt) {
@@ -430,6 +467,63 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
         };
         int restart = -1, done = 0;
         bool gave_up = false;  // the same in every thread
+        // Whether a sum over the lanes' v leaves it open that the SOR stops
+        // (tb_finish_fast's bound).
+        auto open_bound = [&](float v) LES_INLINE {
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const float lb = __fsub_rd(__fmul_rd(v, 0.99609375f), 0x1p-33f);
+            return !(lb >= a.pjuge && lb < 0x1p40f);
+        };
+        // The same for the batch that ends with iteration it, from the words of
+        // all CTAs (the same sum in every CTA), by one warp: the words fetched
+        // into s_words, or polled where one was not there yet.
+        auto words_of = [&](int it) { return a.resid + (size_t)batch_of(it) * a.rstride; };
+        auto open_batch = [&](int it, bool fetched) LES_INLINE {
+            const unsigned t = tag0 + 2u * (unsigned)(it + 1);
+            float v = 0.0f;
+            bool there = fetched;
+            if (fetched)
+#pragma unroll
+                for (int q = 0; q < kResCtas / 32; ++q)
+                    if (lane + 32 * q < ncta) {
+                        const u64 w = s_words[lane + 32 * q];
+                        v += __uint_as_float((unsigned)w);
+                        there = there && (unsigned)(w >> 32) == t;
+                    }
+            if (!__all_sync(0xffffffffu, there)) {
+                v = 0.0f;
+#pragma unroll 1
+                for (int b = lane; b < ncta; b += 32) {
+                    u64 w = word_load(words_of(it) + b);
+                    for (int n = 0; (unsigned)(w >> 32) != t; ++n) {
+                        if (n > kResPolls || *(volatile int *)&s_abort) {
+                            *(volatile int *)&s_abort = 1;
+                            break;
+                        }
+                        w = word_load(words_of(it) + b);
+                    }
+                    v += __uint_as_float((unsigned)w);
+                }
+                __syncwarp();
+            }
+            return open_bound(v);
+        };
+        // At the end of iteration l: the batch that ended two iterations ago, and
+        // the fetch of the one that ended in the last.  With short segments, where
+        // the warps wait more than they issue, by another warp than the one that
+        // sums this CTA's terms (61 x 47 x 35: SOR 161 us, one warp for both 170);
+        // with long ones by the same (150 x 150 x 90: 370, two warps 383).
+        auto look = [&](int l) LES_INLINE {
+            if (l >= 2 && batch_ends(l - 2)) {
+                word_fetch_wait();
+                __syncwarp();
+                if (open_batch(l - 2, true) && lane == 0) s_look[l & 1] = batch_first(l - 2);
+                __syncwarp();
+            }
+            if (l >= 1 && batch_ends(l - 1))
+                for (int b = 2 * lane; b < ncta; b += 64) word_fetch2(s_words + b, words_of(l - 1) + b);
+        };
         // One half-sweep; FIRST: of the attempt (its halo columns came from memory).
         auto sweep = [&](auto Qc, auto EXc, bool first) LES_INLINE {
             if (wedge && !first) receive(decltype(Qc)::value, tag);
@@ -456,17 +550,43 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
             // the others go on (the slots are written again two barriers later)
             float *f = sumf + (l & 1) * blockDim.x;
             f[tid] = act ? fs : 0.0f;  // (idle lanes carry a column's seam values)
-            gave_up = __syncthreads_or(*(volatile int *)&s_abort);
-            if (gave_up) break;
-            if (wid == a.warps - 1) {
-                float v = 0.0f;
-                for (int t = lane; t < (int)blockDim.x; t += 32) v += f[t];
+            // (or the look that ended in this iteration left a stop open: it was
+            // written before the barrier between the half-sweeps, and every CTA's
+            // look finds the same, so all leave the attempt here)
+            if (__syncthreads_or(*(volatile int *)&s_abort | (s_look[(l + 1) & 1] >= 0))) {
+                gave_up = true;
+                break;
+            }
+            if (attempt == 0 && stops) {
+                if (wid == a.warps - 1) {
+                    float v = 0.0f;
+                    for (int t = lane; t < (int)blockDim.x; t += 32) v += f[t];
+                    if (ncta == 1) {
+                        if (open_bound(v) && lane == 0) s_look[l & 1] = l;
+                        continue;
+                    }
 #pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                if (lane == 0) a.resid[(size_t)l * ncta + cta] = v;
+                    for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                    if (lane == 0) {
+                        // the least of the batch, summed over the CTAs, is below each
+                        // iteration's sum (a NaN stays)
+                        if (batch_first(l) < l && !(v < s_min) && v == v) v = s_min;
+                        s_min = v;
+                        if (batch_ends(l) || l == exact_from - 1) word_store(words_of(l) + cta, v, tag);
+                    }
+                    if (SEG >= 40) look(l);
+                } else if (SEG < 40 && wid == a.warps - 2 && ncta > 1) {
+                    look(l);
+                }
             }
         }
-        for (; l < a.itmax && !gave_up; ++l) {
+        word_fetch_wait();
+        if (gave_up) {
+            restart = s_look[(l + 1) & 1];
+            gave_up = restart < 0 || res_grid_barrier(a, ncta, &s_abort);  // all have left the attempt
+            if (tid == 0) s_look[0] = s_look[1] = -1;
+        }
+        for (; l < a.itmax && !gave_up && restart < 0; ++l) {
             fh = flo = 0;
             bad = 0;
             iterate(std::true_type(), l == 0);
@@ -477,18 +597,14 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
             block_fix_sum_any((i128)(((unsigned __int128)fh << 64) | (unsigned __int128)flo), bad, part + cta);
             gave_up = res_grid_barrier(a, ncta, &s_abort);
             if (gave_up) break;
-            if (l == exact_from && attempt == 0 && l > 0) {
-                // every earlier iteration's bound (tb_finish_fast): the first
-                // that does not rule the stop out
+            if (l == exact_from && attempt == 0 && l > 0 && stops) {
+                // the batches whose look is still to come or was not acted on:
+                // the first that does not rule the stop out
                 if (tid == 0) s_stop = INT_MAX;
                 __syncthreads();
-                for (int t = wid; t < l; t += a.warps) {
-                    float v = 0.0f;
-                    for (int b = lane; b < ncta; b += 32) v += __ldcg(&a.resid[(size_t)t * ncta + b]);
-#pragma unroll
-                    for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                    const float lb = __fsub_rd(__fmul_rd(v, 0.99609375f), 0x1p-33f);
-                    if (lane == 0 && !(lb >= a.pjuge && lb < 0x1p40f)) atomicMin(&s_stop, t);
+                for (int t = max(0, l - 3 - kResBatch) + wid; t < l; t += a.warps) {
+                    const bool u = ncta == 1 ? s_look[t & 1] == t : (batch_ends(t) || t == l - 1) && open_batch(t, false);
+                    if (lane == 0 && u) atomicMin(&s_stop, ncta == 1 ? t : batch_first(t));
                 }
                 __syncthreads();
                 if (s_stop != INT_MAX) restart = s_stop;
