@@ -128,8 +128,10 @@ les_status les_step(les_ctx *ctx, int n0, int nsteps);
  * before the next step (run_LES_kernel's per-step wind_profile argument). */
 les_status les_set_wind_profile(les_ctx *ctx, const float *wind_profile);
 /* Waits for the context's work.  LES_ERR_TIMEOUT (here, in les_last_metrics,
- * les_ctx_download and les_ensemble_sync): a bounded wait between the thread
- * blocks of a step's SOR gave up; the state is not that step's. */
+ * les_ctx_download, les_ctx_upload and les_ensemble_sync): a bounded wait
+ * between the thread blocks of a step's SOR gave up; the state is not that
+ * step's.  Reported once; a state uploaded after it steps as in a new
+ * context. */
 les_status les_ctx_sync(les_ctx *ctx);
 les_status les_last_metrics(les_ctx *ctx, les_metrics *m);
 /* The WV_DEBUG sums (velnw.f95:61-68, feedbf.f95:30-36,68-83, the sum(x)
@@ -155,6 +157,9 @@ les_status les_ctx_set_timing(les_ctx *ctx, int nslots);
  * give identical results; odd jp and a just-uploaded p whose ghosts are not
  * boundary-consistent always use the per-colour sweeps. */
 les_status les_ctx_set_sor_path(les_ctx *ctx, int exact);
+/* Diagnostic: polls after which a wait between the thread blocks of the
+ * one-launch SOR gives up (LES_ERR_TIMEOUT); 0: the default, about a second. */
+les_status les_ctx_set_sor_wait(les_ctx *ctx, int polls);
 /* Bounds-checked build (liblesb200_checked.so, compiled with LES_CHECKED):
  * every box index of the time step's kernels is checked against its
  * allocation; an index outside it is counted, the first one's (i, j, k)

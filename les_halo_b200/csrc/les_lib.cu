@@ -212,6 +212,8 @@ struct les_ctx {
     FixPart *d_respart = nullptr;
     unsigned *d_resctl = nullptr;
     int *h_reserr = nullptr, *d_reserr = nullptr;  // host-mapped (res_err_take): a bounded wait of it gave up
+    size_t res_resid = 0;            // bytes of d_resid
+    int res_polls = kResPolls;       // les_ctx_set_sor_wait
     bool cn_uni = false;             // cn2l = cn2s and cn3l = cn3s, one value each
     bool cn1_by_k = false;           // uniform dx, dy: cn1 from a per-k table
     bool p_ghosts_ok = false;        // p's ghosts hold what boundp1/boundp2 give
@@ -862,6 +864,14 @@ void res_err_give(les_ctx *c) {
     c->h_reserr = nullptr;
 }
 
+// Exchange words, bounds and control words as before the first launch.
+les_status res_clear(les_ctx *c) {
+    CK(cudaMemsetAsync(c->d_ll, 0, 2 * c->res.ll_words * sizeof(ulonglong2), c->stream));
+    CK(cudaMemsetAsync(c->d_resid, 0, c->res_resid, c->stream));
+    CK(cudaMemsetAsync(c->d_resctl, 0, 3 * sizeof(unsigned), c->stream));
+    return LES_OK;
+}
+
 // Plan and buffers of the chip-resident SOR, once per context, before the
 // first step is captured.  A grid that does not fit keeps the passes.
 les_status res_setup(les_ctx *c) {
@@ -897,11 +907,9 @@ les_status res_setup(les_ctx *c) {
     c->d_resid = reinterpret_cast<u64 *>(base + ll + rg + part);
     c->d_resctl = reinterpret_cast<unsigned *>(base + ll + rg + part + residp);
     if (!res_err_take(c)) return fail(LES_ERR_NOMEM, "mapped word of the resident SOR");
-    CK(cudaMemsetAsync(c->d_ll, 0, ll, c->stream));
-    CK(cudaMemsetAsync(c->d_resid, 0, resid, c->stream));
-    CK(cudaMemsetAsync(c->d_resctl, 0, 3 * sizeof(unsigned), c->stream));
     c->res = p;
-    return LES_OK;
+    c->res_resid = resid;
+    return res_clear(c);
 }
 
 les_status launch_sor_res(les_ctx *c) {
@@ -920,6 +928,7 @@ les_status launch_sor_res(les_ctx *c) {
     a.c3 = c->h_tables[c->tl.cn3l];
     a.itmax = c->prm.nmaxp;
     a.exact0 = c->sor_fp32_test && c->prm.pjuge < 0x1p40f ? 0 : 1;
+    a.polls = c->res_polls;
     a.pjuge = c->prm.pjuge;
     a.nti = p.nti, a.ntj = p.ntj, a.ti = p.ti, a.tj = p.tj, a.nseg = p.nseg;
     a.pm = p.pm, a.nc = p.nc, a.lch = p.lch, a.warps = p.warps;
@@ -943,11 +952,14 @@ les_status launch_sor_res(les_ctx *c) {
 
 // After a synchronisation: whether a bounded wait of the resident SOR gave
 // up in a step since the last call (p and what follows from it are then
-// not the step's).
+// not the step's).  What the abandoned launch left is cleared here, so that a
+// state uploaded after the report steps from clean words; steps queued before
+// it are void too.
 les_status res_check(les_ctx *c) {
     if (!c->h_reserr || !*(volatile int *)c->h_reserr) return LES_OK;
     *c->h_reserr = 0;
-    CK(cudaMemsetAsync(c->d_resctl, 0, 2 * sizeof(unsigned), c->stream));
+    const les_status s = res_clear(c);
+    if (s != LES_OK) return s;
     CK(cudaStreamSynchronize(c->stream));
     return fail(LES_ERR_TIMEOUT, "SOR: a CTA waited for a neighbour's columns too long; the step is void");
 }
@@ -1400,7 +1412,11 @@ les_status les_ctx_upload(les_ctx *c, const les_host_fields *hf) {
     if (!hf->dx1 || !hf->dy1 || !hf->dzn || !hf->dzs || !hf->dxs || !hf->dys || !hf->cn2l || !hf->cn2s ||
         !hf->cn3l || !hf->cn3s || !hf->cn4l || !hf->cn4s)
         return fail(LES_ERR_BAD_ARG, "metric tables and Poisson coefficients are required");
-    les_status s = scan_inputs(c, hf);
+    // a void step queued before is reported first (and its words cleared)
+    CK(cudaStreamSynchronize(c->stream));
+    les_status s = res_check(c);
+    if (s != LES_OK) return s;
+    s = scan_inputs(c, hf);
     if (s != LES_OK) return s;
     s = build_tables(c, hf, true);
     if (s != LES_OK) return s;
@@ -1522,6 +1538,16 @@ les_status les_ctx_set_sor_path(les_ctx *c, int exact) {
     LES_RANGE("les_ctx_set_sor_path");
     if (!c) return fail(LES_ERR_BAD_ARG, "NULL ctx");
     c->force_exact_sor = exact != 0;
+    return ok();
+}
+
+les_status les_ctx_set_sor_wait(les_ctx *c, int polls) {
+    LES_RANGE("les_ctx_set_sor_wait");
+    if (!c || polls < 0 || polls > kResPolls) return fail(LES_ERR_BAD_ARG, "bad argument");
+    CK(cudaStreamSynchronize(c->stream));
+    c->res_polls = polls ? polls : kResPolls;
+    ++c->table_gen;       // an ensemble's graph holds the limit too
+    drop_step_graphs(c);  // the captured steps hold the old limit
     return ok();
 }
 

@@ -61,8 +61,11 @@
 // 363 -> 377, 257 x 203 x 61 681 -> 711) and nothing where no stop is asked for.
 // Iteration counts, the residual and p are those of exact sums throughout.
 //
-// Every wait is bounded: past kResPolls polls a thread gives up, the CTA
-// returns without writing p, and the context reports LES_ERR_TIMEOUT.
+// Every wait is bounded: past a.polls polls a thread gives up, the CTA
+// returns without writing p, and the context reports LES_ERR_TIMEOUT.  Such a
+// launch leaves words of its own tags behind and does not move ctl[2] on: the
+// words and the control words are zeroed before the next step (res_clear), or
+// that step would take them for its neighbours'.
 #pragma once
 #include "les_sor1.cuh"
 
@@ -72,7 +75,7 @@ namespace {
 typedef unsigned long long u64;
 // a lambda left out of line would move the register window it captures to local memory
 #define LES_INLINE __attribute__((always_inline))
-constexpr int kResPolls = 1 << 20;   // about a second
+constexpr int kResPolls = 1 << 20;   // about a second (ResArgs::polls)
 constexpr int kResList = 64;         // halo columns of one warp (at most two per column)
 constexpr int kResCtas = 160;        // CTAs of a launch, at most
 // Batches of iterations whose FP32 bounds travel as one word: the first four
@@ -106,6 +109,7 @@ struct ResArgs {
     Scal *sc;
     float c2, c3;        // cn2l = cn2s and cn3l = cn3s of every column
     int itmax, exact0;   // iterations; 1: exact sums from the first on
+    int polls;           // of one wait before it gives up
     float pjuge;
     int nti, ntj, ti, tj, nseg, pm, nc, lch, warps;
     int ll_slot;         // words of one slot
@@ -155,7 +159,7 @@ __device__ __forceinline__ bool res_grid_barrier(const ResArgs &a, int ncta, int
             *gen = g0 + 1u;
         } else {
             for (int it = 0; *gen == g0; ++it)
-                if (it > kResPolls || *(volatile int *)s_abort) {
+                if (it > a.polls || *(volatile int *)s_abort) {
                     *(volatile int *)s_abort = 1;
                     break;
                 }
@@ -452,7 +456,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
                     for (int q = 0; q < NE; ++q)
                         ok = ok && (unsigned)(v[q].x >> 32) == t && (unsigned)(v[q].y >> 32) == t;
                     if (ok) break;
-                    if (++it > kResPolls || *(volatile int *)&s_abort) {
+                    if (++it > a.polls || *(volatile int *)&s_abort) {
                         *(volatile int *)&s_abort = 1;
                         break;
                     }
@@ -497,7 +501,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
                 for (int b = lane; b < ncta; b += 32) {
                     u64 w = word_load(words_of(it) + b);
                     for (int n = 0; (unsigned)(w >> 32) != t; ++n) {
-                        if (n > kResPolls || *(volatile int *)&s_abort) {
+                        if (n > a.polls || *(volatile int *)&s_abort) {
                             *(volatile int *)&s_abort = 1;
                             break;
                         }
