@@ -127,11 +127,13 @@ les_status les_step(les_ctx *ctx, int n0, int nsteps);
 /* Replace the external inflow profile wind_profile(1:jp,1:kp) (host array)
  * before the next step (run_LES_kernel's per-step wind_profile argument). */
 les_status les_set_wind_profile(les_ctx *ctx, const float *wind_profile);
-/* Waits for the context's work.  LES_ERR_TIMEOUT (here, in les_last_metrics,
- * les_ctx_download, les_ctx_upload and les_ensemble_sync): a bounded wait
+/* Waits for the context's work.  LES_ERR_TIMEOUT (here and in every call that
+ * waits for the steps queued before it to hand on what they left: metrics,
+ * downloads and uploads, sums, halos, warm-up, phase times, statistics and
+ * restart files, objective and gradients, les_ensemble_sync): a bounded wait
  * between the thread blocks of a step's SOR gave up; the state is not that
- * step's.  Reported once; a state uploaded after it steps as in a new
- * context. */
+ * step's, nor is what the call has written.  Reported once; a state uploaded
+ * after it steps as in a new context. */
 les_status les_ctx_sync(les_ctx *ctx);
 les_status les_last_metrics(les_ctx *ctx, les_metrics *m);
 /* The WV_DEBUG sums (velnw.f95:61-68, feedbf.f95:30-36,68-83, the sum(x)

@@ -258,6 +258,7 @@ float *field_ptr(les_ctx *c, int f) { return c->d_fields + (size_t)f * c->box_el
 les_status launch_sor_tb(les_ctx *c, const TbShape &sh, int niter, int mode, float pjuge, int itmax,
                          bool tuning = false, const SorBufs *bufs = nullptr);
 les_status launch_sor_res(les_ctx *c);
+les_status ctx_wait(les_ctx *c);
 constexpr int kResIters = 4096;  // iterations its residual record holds
 constexpr size_t kResStatic = 2048;  // its static shared memory, at most
 
@@ -964,6 +965,13 @@ les_status res_check(les_ctx *c) {
     return fail(LES_ERR_TIMEOUT, "SOR: a CTA waited for a neighbour's columns too long; the step is void");
 }
 
+// Waits for the context's work: every call that hands on what a step left, or
+// goes on from it, ends in this.
+les_status ctx_wait(les_ctx *c) {
+    CK(cudaStreamSynchronize(c->stream));
+    return res_check(c);
+}
+
 // Process-wide cache of autotuned SOR pass shapes: (ip, jp, kp, SMs) -> shape.
 struct TuneKey {
     int ip, jp, kp, nsm;
@@ -1413,8 +1421,7 @@ les_status les_ctx_upload(les_ctx *c, const les_host_fields *hf) {
         !hf->cn3l || !hf->cn3s || !hf->cn4l || !hf->cn4s)
         return fail(LES_ERR_BAD_ARG, "metric tables and Poisson coefficients are required");
     // a void step queued before is reported first (and its words cleared)
-    CK(cudaStreamSynchronize(c->stream));
-    les_status s = res_check(c);
+    les_status s = ctx_wait(c);
     if (s != LES_OK) return s;
     s = scan_inputs(c, hf);
     if (s != LES_OK) return s;
@@ -1459,7 +1466,7 @@ les_status les_ctx_download(les_ctx *c, les_host_fields *hf) {
         if ((s = download_field(c, f, dst[f])) != LES_OK) return s;
         CK(cudaStreamSynchronize(c->stream));
     }
-    if ((s = res_check(c)) != LES_OK) return s;
+    if ((s = ctx_wait(c)) != LES_OK) return s;
     if (hf->delx1) {
         for (int k = 1; k <= c->prm.kp; ++k) {
             const float *h = c->h_tables.data();
@@ -1482,8 +1489,8 @@ les_status les_ctx_field_sums(les_ctx *c, double *sums) {
         LAUNCH(c, k_field_sum_final, dim3(1), dim3(1024), c->d_part, nb, d_out + f);
     }
     CK(cudaMemcpyAsync(sums, d_out, sizeof(double) * LES_NFIELDS, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    return ok();
+    const les_status s = ctx_wait(c);
+    return s == LES_OK ? ok() : s;
 }
 
 les_status les_ctx_warmup(les_ctx *c, int n) {
@@ -1497,7 +1504,7 @@ les_status les_ctx_warmup(les_ctx *c, int n) {
     if ((s = enqueue_bondv1(c, n, false)) != LES_OK) return s;
     if ((s = enqueue_boundp(c, false)) != LES_OK) return s;
     if ((s = enqueue_velfg_les(c, false)) != LES_OK) return s;
-    CK(cudaStreamSynchronize(c->stream));
+    if ((s = ctx_wait(c)) != LES_OK) return s;
     c->p_ghosts_ok = true;  // ifdata.f95:260-262 applied boundp1, boundp2
     return ok();
 }
@@ -1708,7 +1715,7 @@ les_status les_ctx_set_timing(les_ctx *c, int nslots) {
 les_status les_ctx_phase_times(les_ctx *c, int slot, float *ms, int n) {
     LES_RANGE("les_ctx_phase_times");
     if (!c || !ms || slot < 0 || slot >= c->tslots) return fail(LES_ERR_BAD_ARG, "bad slot");
-    CK(cudaStreamSynchronize(c->stream));
+    if (const les_status s = ctx_wait(c); s != LES_OK) return s;
     // ms[0..7]: consecutive phases between the events; ms[8]: whole step
     for (int w = 0; w < LES_NTEV && w < n; ++w) {
         const int a = (w == LES_NTEV - 1) ? EV_START : w, b = (w == LES_NTEV - 1) ? EV_PAV : w + 1;
@@ -1720,9 +1727,8 @@ les_status les_ctx_phase_times(les_ctx *c, int slot, float *ms, int n) {
 les_status les_ctx_sync(les_ctx *c) {
     LES_RANGE("les_ctx_sync");
     if (!c) return fail(LES_ERR_BAD_ARG, "NULL ctx");
-    CK(cudaStreamSynchronize(c->stream));
-    les_status rs = res_check(c);
-    return rs == LES_OK ? ok() : rs;
+    const les_status s = ctx_wait(c);
+    return s == LES_OK ? ok() : s;
 }
 
 les_status les_last_metrics(les_ctx *c, les_metrics *m) {
@@ -1730,8 +1736,7 @@ les_status les_last_metrics(les_ctx *c, les_metrics *m) {
     if (!c || !m) return fail(LES_ERR_BAD_ARG, "NULL argument");
     Scal s;
     CK(cudaMemcpyAsync(&s, c->d_scal, sizeof s, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (const les_status rs = res_check(c); rs != LES_OK) return rs;
+    if (const les_status rs = ctx_wait(c); rs != LES_OK) return rs;
     m->n = s.n;
     m->sor_iters = s.sor_iters;
     m->sor = s.sor;
@@ -1832,8 +1837,8 @@ static les_status ctx_halo(les_ctx *c, int which, float *buf, int write) {
         LAUNCH(c, k_ctx_halo, dim3(cdiv((long long)n, 256)), dim3(256), c->geo, cv, c->d_stage, d, write);
         if (!write) CK(cudaMemcpyAsync(buf, c->d_stage, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
     }
-    CK(cudaStreamSynchronize(c->stream));
-    return ok();
+    const les_status s = ctx_wait(c);
+    return s == LES_OK ? ok() : s;
 }
 les_status les_ctx_halo_read(les_ctx *c, int which, float *buf) {
     LES_RANGE("les_ctx_halo_read");

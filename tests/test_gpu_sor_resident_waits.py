@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import oracle
-from les_halo_b200 import GpuLes, abi, fields as FL, synthetic_case
+from les_halo_b200 import Ensemble, GpuAdjoint, GpuLes, abi, fields as FL, synthetic_case
 from tests.helpers import assert_bitexact
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +57,89 @@ def test_a_void_step_leaves_nothing_behind(require_gpu, dims, nsteps, at_upload)
     assert_bitexact(got, ref.download(FL.STATE), *dims, FL.STATE)
     assert m["sor_iters"] == ref.metrics()["sor_iters"]
     ref.close()
+
+
+BOX = ((2, 20), (2, 20), (2, 10))
+
+
+def _halo_read(g, adj, tmp):
+    L = abi.lib()
+    buf = np.zeros(L.les_ctx_halo_floats(g.ctx, 0), np.float32)
+    abi.check(L.les_ctx_halo_read(g.ctx, 0, buf.ctypes.data))
+
+
+def _halo_write(g, adj, tmp):
+    L = abi.lib()
+    buf = np.zeros(L.les_ctx_halo_floats(g.ctx, 0), np.float32)
+    abi.check(L.les_ctx_halo_write(g.ctx, 0, buf.ctypes.data))
+
+
+def _phase_times(g, adj, tmp):
+    abi.check(abi.lib().les_ctx_phase_times(g.ctx, 0, (C.c_float * 9)(), 9))
+
+
+def _reverse(g, adj, tmp):
+    adj.zero()
+    adj.seed_tke(-1, BOX, 1.0)
+    adj.step_b(1, 0)
+    adj.read(state=True)
+
+
+# every call that waits for the step and hands something of it on
+CALLS = {
+    "sync": lambda g, adj, tmp: g.sync(),
+    "metrics": lambda g, adj, tmp: g.metrics(),
+    "download": lambda g, adj, tmp: g.download(["u"]),
+    "field_sums": lambda g, adj, tmp: g.field_sums(),
+    "halo_read": _halo_read,
+    "halo_write": _halo_write,
+    "phase_times": _phase_times,
+    "warmup": lambda g, adj, tmp: g.warmup(1),
+    "aveflow_files": lambda g, adj, tmp: g.aveflow(1, 1, 1, 0.0, tmp / "d10", tmp / "d11"),
+    "aveflow_download": lambda g, adj, tmp: (g.aveflow(1, 1, 2), g.aveflow_download()),
+    "write_restart": lambda g, adj, tmp: g.write_restart(tmp / "d20", tmp / "d21"),
+    "adj_tke": lambda g, adj, tmp: adj.tke(-1, BOX),
+    "adj_read": _reverse,
+}
+
+
+@pytest.mark.parametrize("call", CALLS)
+def test_every_reader_reports_a_void_step(require_gpu, call, tmp_path):
+    g = GpuLes(_case((61, 47, 35), 5))
+    adj = GpuAdjoint(g, 2, 10)
+    try:
+        adj.save(0)
+        abi.check(abi.lib().les_ctx_set_timing(g.ctx, 2))
+        _void(g)
+        _times_out(CALLS[call], g, adj, tmp_path)
+        g.sync()  # reported once
+        assert not list(tmp_path.iterdir()), "files of a void step"
+    finally:  # the adjoint before its context
+        adj.close()
+        g.close()
+
+
+def test_refined_metrics_report_a_void_step(require_gpu):
+    g = GpuLes(_case((62, 48, 35), 5))
+    g.warmup(1)
+    g.press_refine_fp64(1, 6, 1e-9)
+    _void(g)
+    _times_out(g.refine_metrics)
+    g.close()
+
+
+def test_an_ensemble_reports_every_void_member(require_gpu):
+    gs = [GpuLes(_case((61, 47, 35), 5)), GpuLes(_case((40, 33, 14), 6)), GpuLes(_case((64, 48, 33), 7))]
+    for g in gs:
+        g.warmup(1)
+    for g in (gs[0], gs[2]):
+        abi.check(abi.lib().les_ctx_set_sor_wait(g.ctx, 1))
+    ens = Ensemble(gs)
+    ens.step(1, 1)
+    _times_out(ens.sync)
+    ens.sync()  # one report for all of them
+    for g in gs:
+        g.sync()
+    ens.close()
+    for g in gs:
+        g.close()
