@@ -853,7 +853,9 @@ bool res_err_take(les_ctx *c) {
         return false;
     }
     *c->h_reserr = 0;
-    return cudaHostGetDevicePointer(&c->d_reserr, c->h_reserr, 0) == cudaSuccess;
+    if (cudaHostGetDevicePointer(&c->d_reserr, c->h_reserr, 0) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
 }
 void res_err_give(les_ctx *c) {
     if (!c->h_reserr) return;
@@ -874,7 +876,8 @@ les_status res_clear(les_ctx *c) {
 }
 
 // Plan and buffers of the chip-resident SOR, once per context, before the
-// first step is captured.  A grid that does not fit keeps the passes.
+// first step is captured.  A grid that does not fit, on the chip or in what is
+// left of the device's memory, keeps the passes.
 les_status res_setup(les_ctx *c) {
     if (c->res_tried) return LES_OK;
     c->res_tried = true;
@@ -898,16 +901,21 @@ les_status res_setup(les_ctx *c) {
                  part = 2 * sizeof(FixPart) * (size_t)n, resid = sizeof(u64) * (size_t)((n + 1) & ~1) * c->prm.nmaxp;
     const size_t residp = (resid + 15) / 16 * 16;
     char *base = nullptr;
+    // a device or host out of memory keeps the passes, which have theirs already
     if (cudaMalloc(&base, ll + rg + part + residp + 3 * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
-        return fail(LES_ERR_NOMEM, "buffers of the resident SOR");
+        return LES_OK;
+    }
+    if (!res_err_take(c)) {
+        res_err_give(c);
+        cudaFree(base);
+        return LES_OK;
     }
     c->d_ll = reinterpret_cast<ulonglong2 *>(base);
     c->d_rg = reinterpret_cast<float4 *>(base + ll);
     c->d_respart = reinterpret_cast<FixPart *>(base + ll + rg);
     c->d_resid = reinterpret_cast<u64 *>(base + ll + rg + part);
     c->d_resctl = reinterpret_cast<unsigned *>(base + ll + rg + part + residp);
-    if (!res_err_take(c)) return fail(LES_ERR_NOMEM, "mapped word of the resident SOR");
     c->res = p;
     c->res_resid = resid;
     return res_clear(c);
