@@ -583,8 +583,9 @@ les_status les_ensemble_step(les_ensemble *ens, int n0, int nsteps);
 les_status les_ensemble_sync(les_ensemble *ens);
 void *les_ensemble_stream(les_ensemble *ens);
 /* The ensemble autotuner's record (after the first les_ensemble_step): the
- * candidates' times in ms per four tuning passes of every member (cap
- * entries at most; -1 where not run), their count and the index chosen.
+ * candidates' times in ms per four tuning passes of every member whose steps
+ * launch passes (cap entries at most; -1 where not run), their count and the
+ * index chosen.
  * Candidate 0: each member's own shape; 1..9: one-iteration passes of
  * (tile rows, k chunks, region rows per warp) (28, 1, 1), (28, 2, 1),
  * (24, 1, 1), (20, 1, 1), (12, 1, 1), (28, 1, 2), (28, 2, 2), (20, 1, 2),

@@ -280,6 +280,11 @@ bool sor_resident(const les_ctx *c) {
     return !sor_per_colour(c) && !c->dd && c->res.seg && c->cn1_by_k && c->cn_uni && c->prm.omega == 1.0f && c->prm.nmaxp >= 1 && c->prm.nmaxp <= kResIters;
 }
 
+// The next step launches SOR passes (the refined press has them in any case).
+bool sor_passes(const les_ctx *c) {
+    return c->ref_outer > 0 || (!sor_per_colour(c) && !sor_resident(c));
+}
+
 void drop_step_graphs(les_ctx *c) {
     for (int gi = 0; gi < 4; ++gi) {
         if (c->graph[gi]) cudaGraphExecDestroy(c->graph[gi]);
@@ -1628,8 +1633,7 @@ les_status les_step(les_ctx *c, int n0, int nsteps) {
             les_status st = res_setup(c);
             if (st != LES_OK) return st;
         }
-        // (the refined press uses the passes too)
-        if (((!exact && !sor_resident(c)) || c->ref_outer > 0) && c->tb.T == 0) {
+        if (sor_passes(c) && c->tb.T == 0) {
             LES_RANGE("sor_autotune");
             les_status st = autotune_sor(c);
             if (st != LES_OK) return st;
