@@ -704,7 +704,8 @@ def run_ours(args):
 
     sor_launch_ms = float(np.mean(phases[:, 5])) if not args.profile else float("nan")
     peak, peak_kind = _peaks()
-    ipl = float(L.les_ctx_sor_iters_per_launch(gpu.ctx))
+    resident = bool(L.les_ctx_sor_resident(gpu.ctx))  # then one launch carries the step's iterations
+    ipl = float(m["sor_iters"]) if resident else float(L.les_ctx_sor_iters_per_launch(gpu.ctx))
     sh = [C.c_int() for _ in range(4)]
     abi.check(L.les_ctx_sor_shape(gpu.ctx, *[C.byref(x) for x in sh]))
     tT, tY, tX, tK = (x.value for x in sh)
@@ -738,7 +739,7 @@ def run_ours(args):
                        "l2": "inputs larger than L2 (19 state fields, 3.5 GB)"},
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm",
-                         "kernel": ("k_sor_colour" if ipl < 1 else "k_sor1p" if rw.value == 2 else
+                         "kernel": ("k_sor_res" if resident else "k_sor_colour" if ipl < 1 else "k_sor1p" if rw.value == 2 else
                                     {1: "k_sor1", 2: "k_sor2"}.get(tT, "k_sor_tb")),
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": traffic,

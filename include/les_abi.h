@@ -183,9 +183,17 @@ enum { LES_RED_CANONICAL = 0, LES_RED_F_RHSAV = 1, LES_RED_F_SOR = 2, LES_RED_F_
        LES_RED_FAITHFUL = 7 };
 les_status les_ctx_set_reduction_mode(les_ctx *ctx, int mode);
 /* SOR iterations one SOR kernel launch of the next step carries: 0.5 for a
- * colour sweep, 1 to 3 for a pass; 1 also for grids whose whole SOR runs in
- * one launch with p on the chip (the pass shapes below then stay 0). */
+ * colour sweep, 1 to 3 for a pass.  Where the whole SOR is one launch
+ * (les_ctx_sor_resident) it answers 1, and that launch carries all of the
+ * step's iterations (les_metrics.sor_iters). */
 float les_ctx_sor_iters_per_launch(les_ctx *ctx);
+/* 1: the next step's SOR is one launch with p kept on the chip (known from the
+ * first step on; the pass shapes below then stay 0), 0: colour sweeps or
+ * passes. */
+int les_ctx_sor_resident(les_ctx *ctx);
+/* Diagnostic: on = 0 makes the following steps run the SOR passes where they
+ * would run it in one launch; on != 0 takes that back.  Results are the same. */
+les_status les_ctx_set_sor_resident(les_ctx *ctx, int on);
 /* Iterations per pass and tile rows the autotuner chose for the
  * multi-iteration SOR (0, 0 before the first step that uses it). */
 les_status les_ctx_sor_tile(les_ctx *ctx, int *iters_per_pass, int *tile_rows);

@@ -205,7 +205,7 @@ struct les_ctx {
     bool xy_pow2 = false;  // every x/y spacing divisor a power of two (build_tables)
     // chip-resident SOR (les_sor_res.cuh), set up before the first step that can use it
     ResPlan res;
-    bool res_tried = false;
+    bool res_tried = false, res_off = false;  // res_off: les_ctx_set_sor_resident
     ulonglong2 *d_ll = nullptr;
     float4 *d_rg = nullptr;
     u64 *d_resid = nullptr;
@@ -275,9 +275,10 @@ bool sor_per_colour(const les_ctx *c) {
 
 // The SOR of the next step runs in one launch with p on the chip
 // (les_sor_res.cuh): wherever it fits and the passes would run, unless
-// LES_SOR_TILE asks for a pass shape.
+// LES_SOR_TILE asks for a pass shape or les_ctx_set_sor_resident for passes.
 bool sor_resident(const les_ctx *c) {
-    return !sor_per_colour(c) && !c->dd && c->res.seg && c->cn1_by_k && c->cn_uni && c->prm.omega == 1.0f && c->prm.nmaxp >= 1 && c->prm.nmaxp <= kResIters;
+    return !sor_per_colour(c) && !c->dd && !c->res_off && c->res.seg && c->cn1_by_k && c->cn_uni &&
+           c->prm.omega == 1.0f && c->prm.nmaxp >= 1 && c->prm.nmaxp <= kResIters;
 }
 
 // The next step launches SOR passes (the refined press has them in any case).
@@ -884,7 +885,7 @@ les_status res_clear(les_ctx *c) {
 // first step is captured.  A grid that does not fit, on the chip or in what is
 // left of the device's memory, keeps the passes.
 les_status res_setup(les_ctx *c) {
-    if (c->res_tried) return LES_OK;
+    if (c->res_tried || c->res_off) return LES_OK;
     c->res_tried = true;
     int dev = 0, coop = 0;
     CK(cudaGetDevice(&dev));
@@ -1552,6 +1553,19 @@ float les_ctx_sor_iters_per_launch(les_ctx *c) {
     const bool exact = sor_per_colour(c);
     if (!exact && sor_resident(c)) return 1.0f;
     return exact ? 0.5f : (float)(c->tb.T ? c->tb.T : 2);
+}
+
+int les_ctx_sor_resident(les_ctx *c) { return c && sor_resident(c) ? 1 : 0; }
+
+les_status les_ctx_set_sor_resident(les_ctx *c, int on) {
+    LES_RANGE("les_ctx_set_sor_resident");
+    if (!c) return fail(LES_ERR_BAD_ARG, "NULL ctx");
+    if (c->res_off == (on == 0)) return ok();
+    CK(cudaStreamSynchronize(c->stream));
+    c->res_off = on == 0;
+    ++c->table_gen;       // an ensemble's graph holds the choice too
+    drop_step_graphs(c);  // the captured steps hold the other one
+    return ok();
 }
 
 les_status les_ctx_set_sor_path(les_ctx *c, int exact) {
