@@ -159,6 +159,10 @@ les_status les_ctx_set_timing(les_ctx *ctx, int nslots);
  * give identical results; odd jp and a just-uploaded p whose ghosts are not
  * boundary-consistent always use the per-colour sweeps. */
 les_status les_ctx_set_sor_path(les_ctx *ctx, int exact);
+/* Diagnostic: planes that one thread block of the momentum kernels marches
+ * (the last block of a column the rest of them); 0: chosen by the grid.
+ * Results are the same. */
+les_status les_ctx_set_mom_planes(les_ctx *ctx, int planes);
 /* Diagnostic: polls after which a wait between the thread blocks of the
  * one-launch SOR gives up (LES_ERR_TIMEOUT); 0: the default, about a second. */
 les_status les_ctx_set_sor_wait(les_ctx *ctx, int polls);

@@ -107,6 +107,7 @@ _SIGS = {
     "les_ctx_set_sor_path": (C.c_int, [_P, C.c_int]),
     "les_ctx_sor_resident": (C.c_int, [_P]),
     "les_ctx_set_sor_resident": (C.c_int, [_P, C.c_int]),
+    "les_ctx_set_mom_planes": (C.c_int, [_P, C.c_int]),
     "les_ctx_set_sor_wait": (C.c_int, [_P, C.c_int]),
     "les_ctx_set_reduction_mode": (C.c_int, [_P, C.c_int]),
     "les_bounds_violations": (C.c_int, [C.POINTER(C.c_ulonglong), _I]),

@@ -195,6 +195,7 @@ struct les_ctx {
     bool rhs_raw = false;  // interior of rhs holds values before the rhsav subtraction
     int red_gx = 0, red_gy = 0, red_nk = 0, red_kchunk = 0;
     int nsm = 148;  // SMs of the context's device
+    int mom_planes = 0;  // les_ctx_set_mom_planes (0: mom_kchunk's choice)
     int last_n = 0;
     std::vector<float *> extra;      // scratch boxes of the per-routine entries
     const float *cn1_box = nullptr;  // caller's cn1 (per-routine press only)
@@ -493,7 +494,9 @@ int mom_kchunk(int km, long long tiles, int cap) {
 les_status enqueue_velfg_les(les_ctx *c, bool adam) {
     const Geo &g = c->geo;
     const long long tiles = (long long)cdiv(g.im, kMX) * cdiv(g.jm, kMY);
-    const int kc1 = mom_kchunk(g.km, tiles, c->nsm * kMom1PerSM), kc2 = mom_kchunk(g.km, tiles, c->nsm * kMom2PerSM);
+    const int own = std::min(c->mom_planes, g.km);
+    const int kc1 = own ? own : mom_kchunk(g.km, tiles, c->nsm * kMom1PerSM),
+              kc2 = own ? own : mom_kchunk(g.km, tiles, c->nsm * kMom2PerSM);
     const dim3 mg(cdiv(g.im, kMX), cdiv(g.jm, kMY), cdiv(g.km, kc1));
     const dim3 mg2(mg.x, mg.y, cdiv(g.km, kc2));
     const bool band = g.jm >= kBH;  // the staged band must not wrap onto itself
@@ -1572,6 +1575,16 @@ les_status les_ctx_set_sor_path(les_ctx *c, int exact) {
     LES_RANGE("les_ctx_set_sor_path");
     if (!c) return fail(LES_ERR_BAD_ARG, "NULL ctx");
     c->force_exact_sor = exact != 0;
+    return ok();
+}
+
+les_status les_ctx_set_mom_planes(les_ctx *c, int planes) {
+    LES_RANGE("les_ctx_set_mom_planes");
+    if (!c || planes < 0) return fail(LES_ERR_BAD_ARG, "bad argument");
+    CK(cudaStreamSynchronize(c->stream));
+    c->mom_planes = planes;
+    ++c->table_gen;       // an ensemble's graph holds the cut too
+    drop_step_graphs(c);  // the captured steps hold the old one
     return ok();
 }
 
