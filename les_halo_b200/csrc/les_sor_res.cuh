@@ -4,8 +4,11 @@
 // A pass over HBM (k_sor1, k_sor1p) costs one march over the planes of a k
 // chunk, about 1 us a plane: 23 us a pass at 150 x 150 x 90, where its bytes
 // take 4, and 11 us at 24 x 20 x 16.  A grid whose p and rhs fit in the SMs'
-// registers and shared memory (about 3 million cells) need not move them
-// between iterations at all, so here
+// registers and shared memory need not move them between iterations at all.
+// What fits is a matter of tiles, segments and threads, not of cells alone
+// (res_plan): 257 x 203 x 61 does with 3.18 million cells, 195 x 195 x 80 with
+// 3.04 does not (its columns are two segments of 40 planes, too many threads, or
+// pad to 128).  So here
 //   - a CTA owns a ti x tj tile of (i,j) columns, all km planes; the launch is
 //     cooperative, one CTA per SM, and runs every iteration of the step;
 //   - a thread owns one column's segment of SEG planes, its p in registers;
@@ -20,21 +23,24 @@
 //   - a tile's edge columns are sent to the neighbouring tile's CTA after the
 //     half-sweep that updated them, as 64-bit words {value, tag} written and
 //     polled with relaxed loads and stores: the word that arrives is its own
-//     flag, so an exchange costs one trip through L2 and no fence.  The edge
+//     flag (the method of NCCL's low-latency protocol), so an exchange costs one
+//     trip through L2 and no fence.  The edge
 //     columns are the first of each class, so only their warps wait; the other
 //     warps work meanwhile.  Two slots per word suffice: a CTA sends
 //     half-sweep s+2 only after it has received s+1 from the same neighbour
 //     column, which that column sent after it had read s.
-// What bounds it: at 150 x 150 x 90 a half-sweep takes 7.1 thousand cycles, most
-// of it the edge warps' chain.  Clocked when a word was still polled before the
-// others were read (7.5 in all): 3.4 until the neighbours' words are there, 2.5
-// of updates, 0.8 of sends; the other warps' updates, 3.1 (shared memory: 27
-// wavefronts per four updates of a warp), run beside it.
-// With one CTA (24 x 20 x 16) nothing is exchanged and a half-sweep takes 2.2.
+// What bounds it: latency.  At 150 x 150 x 90 a half-sweep takes 3.7 us, 6.7
+// thousand cycles, with 12 warps an SM of which 29% of the issue slots are used;
+// the warps wait at the CTA's barrier for those with edge columns (3.7 cycles per
+// issue), for shared memory (1.9), for the neighbours' words (1.4) and for
+// instructions (0.7: the unrolled loop is larger than the cache).  51 shared-memory
+// wavefronts per four updates of a warp, exchange and bounds included.
+// With one CTA (24 x 20 x 16) nothing is exchanged and a half-sweep takes 1.1 us.
 // Measured, the SOR of a step (50 iterations), passes -> here: 24 x 20 x 16
-// 585 -> 119 us, 61 x 47 x 35 607 -> 162, 150 x 150 x 90 1226 -> 377,
-// 257 x 203 x 61 1618 -> 711.  Packed two-wide FP32 instructions (18% fewer
-// instructions) gave nothing, and need a -0 the assembler cannot see: it
+// 585 -> 119 us, 61 x 47 x 35 607 -> 160, 150 x 150 x 90 1226 -> 373,
+// 257 x 203 x 61 1618 -> 720.  Every segment length spills (12 to 232 bytes of
+// stores): its p fills the registers.  Packed two-wide FP32 instructions (18%
+// fewer instructions) gave nothing, and need a -0 the assembler cannot see: it
 // contracts a packed multiply and add whatever --fmad says.
 //
 // Ghosts (press.f95:87-115 followed through, les_sor_tb.cuh): the i and k
@@ -57,8 +63,11 @@
 // -> while it runs; the passes: 24 x 20 x 16 167 -> 79 us; 220, 61 x 47 x 35
 // 235 -> 118; 235, 150 x 150 x 90 529 -> 271; 352, 257 x 203 x 61 927 -> 380; 440;
 // after 10 of 1000 at 150 x 150 x 90 6132 -> 272; 1428).  The looks cost 0 to 4.5%
-// of an SOR that runs to its cap (61 x 47 x 35 161 -> 162 us, 150 x 150 x 90
-// 363 -> 377, 257 x 203 x 61 681 -> 711) and nothing where no stop is asked for.
+// of an SOR that runs to its cap (61 x 47 x 35 160 -> 160 us, 150 x 150 x 90
+// 365 -> 373, 257 x 203 x 61 688 -> 720) and nothing where no stop is asked for.
+// A stop that is only nearly reached (residuals within 4x of the threshold at the
+// cap) leaves a batch open early and sums the rest exactly: 150 x 150 x 90 770 us,
+// 257 x 203 x 61 1390, still below the passes' 1220 and 1600.
 // Iteration counts, the residual and p are those of exact sums throughout.
 //
 // Every wait is bounded: past a.polls polls a thread gives up, the CTA
@@ -180,6 +189,13 @@ template <int SEG, bool RG>
 __global__ void __launch_bounds__(res_threads(SEG), 1)
     k_sor_res(Geo g, ResArgs a, const __grid_constant__ TbKCoef kq) {
     constexpr int H = SEG / 2, NG = SEG / 8, NE = SEG / 4, CS = SEG + 4;
+    // Long segments unroll to more code than the instruction cache keeps, so what
+    // runs between iterations is fetched anew each time: there the bounds are
+    // summed once per batch and their loops stay rolled (150 x 150 x 90: SOR to
+    // its cap 391 -> 371 us, 257 x 203 x 61 736 -> 719).  Short ones wait for the
+    // latencies of a rolled loop instead (24 x 20 x 16: 119 -> 127).
+    constexpr bool LONG = SEG >= 40;
+    constexpr int UL = LONG ? 1 : 32;  // unrolling of those loops
     extern __shared__ float4 rsm4[];
     __shared__ int s_abort, s_cnt[4], s_stop, s_look[2];
     __shared__ float s_min;
@@ -350,6 +366,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
         __syncthreads();
 
         float fs = 0.0f;       // FP32 sum of reltmp^2
+        float fm = 0.0f;       // its least in the batch (LONG)
         u64 fh = 0, flo = 0;   // exact sum
         int bad = 0;
         // One half-sweep of the thread's planes of parity Q, sent with tag t;
@@ -474,7 +491,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
         // Whether a sum over the lanes' v leaves it open that the SOR stops
         // (tb_finish_fast's bound).
         auto open_bound = [&](float v) LES_INLINE {
-#pragma unroll
+#pragma unroll UL
             for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             const float lb = __fsub_rd(__fmul_rd(v, 0.99609375f), 0x1p-33f);
             return !(lb >= a.pjuge && lb < 0x1p40f);
@@ -488,7 +505,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
             float v = 0.0f;
             bool there = fetched;
             if (fetched)
-#pragma unroll
+#pragma unroll UL
                 for (int q = 0; q < kResCtas / 32; ++q)
                     if (lane + 32 * q < ncta) {
                         const u64 w = s_words[lane + 32 * q];
@@ -526,6 +543,7 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
                 __syncwarp();
             }
             if (l >= 1 && batch_ends(l - 1))
+#pragma unroll UL
                 for (int b = 2 * lane; b < ncta; b += 64) word_fetch2(s_words + b, words_of(l - 1) + b);
         };
         // One half-sweep; FIRST: of the attempt (its halo columns came from memory).
@@ -550,10 +568,14 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
         for (; l < exact_from; ++l) {
             fs = 0.0f;
             iterate(std::false_type(), l == 0);
-            // this iteration's FP32 terms: summed by the CTA's last warp while
-            // the others go on (the slots are written again two barriers later)
+            // this iteration's FP32 terms (LONG: each thread's least of the batch's
+            // iterations, whose sum is below the sum of each; a NaN stays): summed by
+            // the CTA's last warp while the others go on (the slots are written again
+            // two barriers later)
+            const bool ends = batch_ends(l) || l == exact_from - 1, sums = !LONG || ends;
             float *f = sumf + (l & 1) * blockDim.x;
-            f[tid] = act ? fs : 0.0f;  // (idle lanes carry a column's seam values)
+            if (LONG && (batch_first(l) == l || fs < fm || fs != fs)) fm = fs;
+            if (sums) f[tid] = act ? (LONG ? fm : fs) : 0.0f;  // (idle lanes carry a column's seam values)
             // (or the look that ended in this iteration left a stop open: it was
             // written before the barrier between the half-sweeps, and every CTA's
             // look finds the same, so all leave the attempt here)
@@ -563,23 +585,32 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
             }
             if (attempt == 0 && stops) {
                 if (wid == a.warps - 1) {
-                    float v = 0.0f;
-                    for (int t = lane; t < (int)blockDim.x; t += 32) v += f[t];
-                    if (ncta == 1) {
-                        if (open_bound(v) && lane == 0) s_look[l & 1] = l;
-                        continue;
+                    if (sums) {
+                        float v = 0.0f;
+                        if (LONG) {
+#pragma unroll 1
+                            for (int t = lane; t < (int)blockDim.x; t += 32) v += f[t];
+                        } else {
+                            for (int t = lane; t < (int)blockDim.x; t += 32) v += f[t];
+                        }
+                        if (ncta == 1) {
+                            if (open_bound(v) && lane == 0) s_look[l & 1] = LONG ? batch_first(l) : l;
+                            continue;
+                        }
+#pragma unroll UL
+                        for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                        if (lane == 0) {
+                            // the least of the batch, summed over the CTAs, is below each
+                            // iteration's sum (a NaN stays)
+                            if (!LONG) {
+                                if (batch_first(l) < l && !(v < s_min) && v == v) v = s_min;
+                                s_min = v;
+                            }
+                            if (ends) word_store(words_of(l) + cta, v, tag);
+                        }
                     }
-#pragma unroll
-                    for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                    if (lane == 0) {
-                        // the least of the batch, summed over the CTAs, is below each
-                        // iteration's sum (a NaN stays)
-                        if (batch_first(l) < l && !(v < s_min) && v == v) v = s_min;
-                        s_min = v;
-                        if (batch_ends(l) || l == exact_from - 1) word_store(words_of(l) + cta, v, tag);
-                    }
-                    if (SEG >= 40) look(l);
-                } else if (SEG < 40 && wid == a.warps - 2 && ncta > 1) {
+                    if (LONG && ncta > 1) look(l);
+                } else if (!LONG && wid == a.warps - 2 && ncta > 1) {
                     look(l);
                 }
             }
@@ -607,8 +638,9 @@ __global__ void __launch_bounds__(res_threads(SEG), 1)
                 if (tid == 0) s_stop = INT_MAX;
                 __syncthreads();
                 for (int t = max(0, l - 3 - kResBatch) + wid; t < l; t += a.warps) {
-                    const bool u = ncta == 1 ? s_look[t & 1] == t : (batch_ends(t) || t == l - 1) && open_batch(t, false);
-                    if (lane == 0 && u) atomicMin(&s_stop, ncta == 1 ? t : batch_first(t));
+                    const bool u = ncta == 1 ? t == l - 1 && s_look[t & 1] >= 0
+                                             : (batch_ends(t) || t == l - 1) && open_batch(t, false);
+                    if (lane == 0 && u) atomicMin(&s_stop, ncta == 1 ? s_look[t & 1] : batch_first(t));
                 }
                 __syncthreads();
                 if (s_stop != INT_MAX) restart = s_stop;
