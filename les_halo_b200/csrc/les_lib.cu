@@ -795,8 +795,8 @@ les_status set_tb_smem_attrs() {
 // least cost of a half-sweep is taken, in cycles: 15 + 2.25 SEG per warp (what
 // its instructions and shared-memory words take), at least 1500 when columns
 // are exchanged (the trip through L2), and 8 for each row and column of a tile's
-// edge.  Measured against every segment length: the plan taken is the fastest,
-// or within 2% of it, at 24 x 20 x 16 (16 planes: 114 us; 8: 135, 24: 130, 32:
+// edge.  Measured against every segment length (without the looks at the stop
+// bounds): the plan taken is the fastest, or within 2% of it, at 24 x 20 x 16 (16 planes: 114 us; 8: 135, 24: 130, 32:
 // 233), 61 x 47 x 35 (8: 159; 16: 178, 24: 206, 64: 300) and 150 x 150 x 90 (48:
 // 362; 24: 438, 32: 364, 64: 607).
 ResPlan res_plan(int ip, int jp, int kp, int nsm, size_t smem_max) {
